@@ -14,6 +14,7 @@ enum : uint32_t {
     DEVERR_TILE_OVERFLOW = 1u << 1,     // more particles in a tile than staged
     DEVERR_BAD_KEY = 1u << 2,           // a key outside the declared key range
     DEVERR_TMA_TIMEOUT = 1u << 3,       // a TMA copy's mbarrier wait gave up
+    DEVERR_GRID_TIMEOUT = 1u << 4,      // a grid-wide reduction of the resident pressure solve gave up
 };
 
 // Upper bound on polls of a look-back status word before giving up.  The

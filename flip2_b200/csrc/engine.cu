@@ -211,6 +211,9 @@ static int dev_err_eval(flip_engine* e) {
     E_CUDA(cudaMemsetAsync(e->d_err, 0, sizeof(uint32_t), e->stream));
     return e->fail(FLIP_ERR_TIMEOUT, (w & DEVERR_TMA_TIMEOUT)
                                          ? "a TMA copy of G2P timed out; the particles of this step are invalid"
+                                     : (w & DEVERR_GRID_TIMEOUT)
+                                         ? "a grid-wide reduction of the pressure solve timed out; the pressure of this "
+                                           "step is invalid"
                                          : "a decoupled look-back wait of the sort or scan timed out; the binning of "
                                            "this step is invalid");
 }
@@ -406,6 +409,12 @@ extern "C" int flip_set_domain(flip_engine* e, double nx, double ny, double nz, 
         add((void**)&e->d_rec, sizeof(SolveRecord));
         add((void**)&e->d_frame, sizeof(FrameState));
         add((void**)&e->pcg.partials, sizeof(double) * 4 * kPcgBlocks);
+        e->pcg.ctas = (uint32_t)std::min<uint64_t>(std::min(e->sms, kResidentMaxCtas), (e->ntiles_total + 3) / 4);
+        e->pcg.mail_tiles = (uint32_t)std::min<uint64_t>(e->ntiles_total, kResidentTiles * e->pcg.ctas);
+        add((void**)&e->pcg.slots, 8 * kPcgSlotWords * 4 * (size_t)e->pcg.ctas);
+        add((void**)&e->pcg.epoch, sizeof(uint32_t));
+        add((void**)&e->pcg.far, e->ntiles_total > kResidentNoFar * e->pcg.ctas ? 4 * 768 * (size_t)e->pcg.mail_tiles : 0);
+        add((void**)&e->pcg.mail, 8 * 2 * 6 * 64 * (size_t)e->pcg.mail_tiles);
     }
     size_t total = 0;
     for (auto& pr : plan) total += al(pr.second ? pr.second : 1);
@@ -1189,6 +1198,16 @@ static int run_plain_host(flip_engine* e, int chunk, int max_iter) {
     return FLIP_OK;
 }
 
+// the resident solve and its state; done = 0: it left the solve to the loop
+static int run_resident(flip_engine* e, int chunk, int max_iter) {
+    E_TRY(nat_launch_pcg_resident(e->node_keys, e->d_counts, e->D, e->pcg, chunk, loop_limit(max_iter, chunk), e->d_err, e->stream));
+    E_CUDA(cudaMemcpyAsync(e->h_state, e->pcg.st, sizeof(PcgState), cudaMemcpyDeviceToHost, e->stream));
+    E_TRY(dev_err_fetch(e));
+    E_CUDA(cudaStreamSynchronize(e->stream));
+    e->launches += 1;
+    return dev_err_eval(e);
+}
+
 // Solve A x = b on the occupied tiles.  U: face velocities giving b = -div U,
 // or nullptr when b is already in pcg.b.  method 1 runs learned FPCG first and,
 // if it stops without meeting tol (iteration cap or a non-positive r.z),
@@ -1262,11 +1281,14 @@ static int nat_solve(flip_engine* e, const float* const* U, int method, double t
                                    e->type, e->pcg, e->stream, w ? e->cell_prev : nullptr));
         e->launches += w ? 2 : 1;
         if (method == 0) E_TRY(e->mark(9));
-        if (host_solve_loop()) {
-            E_TRY(run_plain_host(e, chunk, max_plain));
-        } else {
-            E_TRY(nat_pcg_graph(e, chunk, max_plain));
-            E_TRY(run_loop(e, e->pcg_graph, 2u * (uint32_t)chunk + 1u));
+        E_TRY(run_resident(e, chunk, max_plain));
+        if (e->h_state->done == 0) {  // more tiles than the chip holds
+            if (host_solve_loop()) {
+                E_TRY(run_plain_host(e, chunk, max_plain));
+            } else {
+                E_TRY(nat_pcg_graph(e, chunk, max_plain));
+                E_TRY(run_loop(e, e->pcg_graph, 2u * (uint32_t)chunk + 1u));
+            }
         }
         E_TRY(nat_launch_solve_record(e->d_rec, e->pcg.st, 0, method == 0 ? 0 : 1, 0, e->stream));
         const PcgState& s = *e->h_state;
@@ -1419,13 +1441,14 @@ static int cap_body(flip_engine* e, cudaGraph_t body, Fn fn) {
 }
 // a WHILE loop of chunks: body() then the loop control kernel; the
 // condition is set to 1 by a kernel before the node, so the loop also runs
-// when it sits inside another loop's body
+// when it sits inside another loop's body (unless_done: to 0 where that
+// state says the solve is done)
 template <class Fn>
-static int cap_loop(flip_engine* e, int limit, Fn body) {
+static int cap_loop(flip_engine* e, int limit, Fn body, const PcgState* unless_done = nullptr) {
     cudaGraphConditionalHandle h;
     cudaGraph_t g = nullptr;
     E_TRY(cap_handle(e, 1u, &h));
-    E_TRY(nat_launch_cond_set(h, 1u, e->stream));
+    E_TRY(nat_launch_cond_set(h, 1u, e->stream, unless_done));
     E_TRY(cap_cond_node(e, cudaGraphCondTypeWhile, h, &g));
     return cap_body(e, g, [&]() {
         E_TRY(body());
@@ -1445,6 +1468,10 @@ static int cap_mg_chunk(flip_engine* e, int chunk, bool network) {
     }
     return FLIP_OK;
 }
+// the box has no more tiles than the resident solve holds
+static bool resident_always(flip_engine* e) {
+    return e->ntiles_total <= (uint64_t)kResidentTiles * e->pcg.ctas;
+}
 // Jacobi-PCG from a fresh state: b from U (nullptr: already in pcg.b),
 // warm: from the previous solution where the device flag allows
 static int cap_plain_solve(flip_engine* e, const float* const* U, bool warm, int stage) {
@@ -1453,7 +1480,9 @@ static int cap_plain_solve(flip_engine* e, const float* const* U, bool warm, int
     E_TRY(nat_launch_state_init(e->pcg.st, e->P.pcg_tol, e->P.pcg_max_iter, e->P.true_residual_every, 0, e->stream));
     E_TRY(nat_launch_pcgw_init(e->node_keys, e->d_counts, e->grid_tiles, e->d_counts + 1, e->D, U ? U : nullU, e->type,
                                e->pcg, e->stream, warm ? e->cell_prev : nullptr));
-    E_TRY(cap_loop(e, loop_limit(e->P.pcg_max_iter, chunk), [&]() { return cap_plain_chunk(e, chunk); }));
+    const int limit = loop_limit(e->P.pcg_max_iter, chunk);
+    E_TRY(nat_launch_pcg_resident(e->node_keys, e->d_counts, e->D, e->pcg, chunk, limit, e->d_err, e->stream));
+    if (!resident_always(e)) E_TRY(cap_loop(e, limit, [&]() { return cap_plain_chunk(e, chunk); }, e->pcg.st));
     return nat_launch_solve_record(e->d_rec, e->pcg.st, 0, stage, 1, e->stream);
 }
 // the pressure solve of a captured step (pressure_method 0 or 2)

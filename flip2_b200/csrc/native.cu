@@ -1639,9 +1639,11 @@ int nat_launch_solve_record(SolveRecord* rec, PcgState* st, int flexible, int st
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-__global__ void cond_set_kernel(cudaGraphConditionalHandle h, unsigned int v) { cudaGraphSetConditional(h, v); }
-int nat_launch_cond_set(cudaGraphConditionalHandle h, unsigned int v, cudaStream_t s) {
-    cond_set_kernel<<<1, 1, 0, s>>>(h, v);
+__global__ void cond_set_kernel(cudaGraphConditionalHandle h, unsigned int v, const PcgState* st) {
+    cudaGraphSetConditional(h, st && st->done ? 0u : v);
+}
+int nat_launch_cond_set(cudaGraphConditionalHandle h, unsigned int v, cudaStream_t s, const PcgState* st) {
+    cond_set_kernel<<<1, 1, 0, s>>>(h, v, st);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }

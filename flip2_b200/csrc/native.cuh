@@ -39,6 +39,13 @@ constexpr double kFlexStall = 0.81;
 constexpr int kPcgBlocks = 592;        // 148 SMs x 4 CTAs of 512 threads
 constexpr int kPcgUpdateBlocks = 592;  // 148 SMs x 4 CTAs of 256 threads (a warp per half tile, 10 loads in flight a lane)
 
+// The resident solve (pcg_resident.cu): tiles a CTA can hold, CTAs at most,
+// and the words of one reader's packets of sums (a line from up to 32 CTAs).
+constexpr int kResidentTiles = 88;
+constexpr int kResidentNoFar = 29;  // tiles a CTA whose faces always have room on the chip
+constexpr int kResidentMaxCtas = 160;
+constexpr int kPcgSlotWords = 512;
+
 // PCG vectors on the tile-blocked slots.  The solution is x + xg: x in FP64
 // holds everything up to the last true-residual check, xg (FP32) the
 // increments since then.  An FP32 solution alone bounds the attainable true
@@ -56,6 +63,12 @@ struct PcgBuffers {
     uint32_t* tcoord;  // packed tile coordinates of the occupied tiles
     PcgState* st;
     double* partials;  // [4][kPcgBlocks]
+    uint32_t ctas;     // CTAs of the resident solve: one per SM, and one per four tiles at most
+    unsigned long long* slots;  // its packets, [2][2][ctas][kPcgSlotWords]
+    uint32_t* epoch;   // the last tag the resident solve used
+    float* far;        // its faces without room on the chip: 768 floats a tile
+    unsigned long long* mail;  // its mailboxes: [2][mail_tiles][6][64] tagged words
+    uint32_t mail_tiles;
     // device flag of the warm start (optional): the previous solve converged,
     // so its solution may start this one; 0 makes a warm-start launch cold
     const int* warm_ok;
@@ -191,6 +204,14 @@ int nat_launch_pcgw_iteration(const uint32_t* tiles, const uint32_t* d_ntiles, c
                               cudaStream_t s);
 int nat_launch_pcgw_check(const uint32_t* tiles, const uint32_t* d_ntiles, const NatDims& D, PcgBuffers& B,
                           cudaStream_t s);
+// the whole plain solve after nat_launch_pcgw_init in one cooperative kernel,
+// for at most kResidentTiles tiles per CTA: the
+// iterations in chunks of `chunk`, the true-residual checks between chunks,
+// at most `limit` chunks.  With more tiles it returns at once and leaves
+// st->done 0; a reduction that gives up sets DEVERR_GRID_TIMEOUT in *err
+// and st->done 5.
+int nat_launch_pcg_resident(const uint32_t* tiles, const uint32_t* d_ntiles, const NatDims& D, PcgBuffers& B, int chunk,
+                            int limit, uint32_t* err, cudaStream_t s);
 // end of a loop chunk inside a conditional WHILE graph node: continue while
 // the solve is not done and fewer than limit chunks have run
 int nat_launch_loop_ctl(cudaGraphConditionalHandle h, PcgState* st, int limit, cudaStream_t s);
@@ -202,8 +223,8 @@ int nat_launch_state_init(PcgState* st, double tol, int max_iter, int true_every
 // stage 1 after the Jacobi-PCG restart; captured: the solve ran inside a
 // captured step (its loop chunks count towards the step's launches)
 int nat_launch_solve_record(SolveRecord* rec, PcgState* st, int flexible, int stage, int captured, cudaStream_t s);
-// sets a conditional node's condition value
-int nat_launch_cond_set(cudaGraphConditionalHandle h, unsigned int v, cudaStream_t s);
+// sets a conditional node's condition value (st: to 0 where the solve is done)
+int nat_launch_cond_set(cudaGraphConditionalHandle h, unsigned int v, cudaStream_t s, const PcgState* st = nullptr);
 // condition of a conditional IF node: the flexible solve did not converge
 int nat_launch_fallback_cond(cudaGraphConditionalHandle h, const PcgState* st, cudaStream_t s);
 // one sub-step of a captured frame: dt = min(max_dt, Courant limit from

@@ -411,7 +411,8 @@ typedef struct {
                                 flip_solve_frame, generateVoxels, the end of each
                                 native pressure solve -- also returns as
                                 FLIP_ERR_TIMEOUT; bit 2: a tensor-core wait of the
-                                learned preconditioner timed out)                */
+                                learned preconditioner timed out; bit 4: a
+                                grid-wide exchange of the pressure solve)        */
     uint32_t launches;       /* kernels this engine launched since creation      */
     uint64_t solves;         /* NATIVE: pressure solves since setDomain           */
     uint64_t fallbacks;      /* NATIVE: of those, flexible solves that missed tol
