@@ -146,117 +146,379 @@ __device__ __forceinline__ RefLocal ref_particle_local(const double* px, const d
     return r;
 }
 
-// getNumberVoxelsUsedPerNode (particles.cu:88-190): mask + count per node.
-// A warp per node (kVoxWarps nodes per CTA): the 512 solid tests as 16
-// ballots (none for a tile away from the domain faces, whose tests all
-// fail), then the node's particles in order, the 64 points of a particle's
-// 4 x 4 x 4 stencil spread over the lanes (two each); a lane loads and
-// prepares one particle of each round of 32, so the loads overlap.  The tests
-// and their arithmetic are the reference's; only the work is spread.  Its
-// loops run x from sx - 2 while (unsigned) x < sx + 2, so a stencil
-// coordinate below 2 on any axis leaves a particle without marks, and points
-// outside the 8^3 tile never mark: both are tested before the distances.
+// The voxels of a particle's stencil in the tile, one word per z plane (bit
+// x + 8 y), for the planes sz - 1, sz, sz + 1.
+//
+// The reference tests 4 x 4 x 4 points at three offsets with FP64 distances.
+// In units of the voxel, f = l / scw - s in [0, 1): a point k = -2 .. 1 voxels
+// away lies at f - k or, with the half-voxel offset, f - k + 1/2 on each axis,
+// so the column k = -2 is never nearer than the radius 2 and 27 points
+// remain.  Their distances are taken in FP32: with f rounded once, every
+// square and sum stays within 5e-6 of the exact value, so a squared distance
+// at least 1e-5 away from 4 decides as the reference's FP64 test does.  The
+// column k = -2 counts with its smallest distance, 4 f + (f' - 1/2)^2 +
+// (f'' - 1/2)^2 above 4.  False (one particle in about 10^4): a distance
+// nearer to 4 than that, or a position outside the root cell; the caller
+// then runs the reference's own test.
+//
+// FP64 tests of all 64 points by a warp per particle took 33 ms for 64M
+// particles in 29.5M nodes.
+__device__ __forceinline__ bool ref_marks(double qx, double qy, double qz, uint32_t sx, uint32_t sy, uint32_t sz,
+                                          unsigned long long (&plane)[3]) {
+    const float fx = (float)(qx - (double)sx), fy = (float)(qy - (double)sy), fz = (float)(qz - (double)sz);
+    const float kNear = 1e-5f;
+    if (sx - 2u > 4u || sy - 2u > 4u || sz - 2u > 4u) return false;
+    // squares of f + 1, f, f - 1 (a) and of those plus 1/2 (b), k = -1, 0, 1
+    float ax[3], bx[3], ay[3], by[3], az[3], bz[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float o = 1.0f - (float)k;
+        ax[k] = (fx + o) * (fx + o) - 4.0f;
+        bx[k] = (fx + o + 0.5f) * (fx + o + 0.5f) - 4.0f;
+        ay[k] = (fy + o) * (fy + o);
+        by[k] = (fy + o + 0.5f) * (fy + o + 0.5f);
+        az[k] = (fz + o) * (fz + o);
+        bz[k] = (fz + o + 0.5f) * (fz + o + 0.5f);
+    }
+    const float hx = (fx - 0.5f) * (fx - 0.5f), hy = (fy - 0.5f) * (fy - 0.5f), hz = (fz - 0.5f) * (fz - 0.5f);
+    float near = fminf(4.0f * fx + (hy + hz), fminf(4.0f * fy + (hx + hz), 4.0f * fz + (hx + hy)));
+    const uint32_t shift = (sx - 1u) + 8u * (sy - 1u);
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+        uint32_t bits = 0;  // nine sign bits, the last pushed lowest
+#pragma unroll
+        for (int y = 2; y >= 0; --y) {
+            const float p = by[y] + bz[z], q = fminf(ay[y] + bz[z], by[y] + az[z]);
+#pragma unroll
+            for (int x = 2; x >= 0; --x) {
+                const float d = fminf(ax[x] + p, bx[x] + q);
+                near = fminf(near, fabsf(d));
+                bits = __funnelshift_l(__float_as_uint(d), bits, 1);
+            }
+        }
+        plane[z] = (unsigned long long)((bits & 7u) | ((bits & 0x38u) << 5) | ((bits & 0x1C0u) << 10)) << shift;
+    }
+    return near > kNear;
+}
+
+// what the particles of one node share: the node's corner and the voxel size
+struct RefNode {
+    double neg[3], corner[3], scw, R, lo, hi;
+};
+__device__ __forceinline__ RefNode ref_node(uint32_t key, const flip_grid& g) {
+    RefNode N;
+    uint32_t gx, gy, gz;
+    ref_decompose(key, g, gx, gy, gz);
+    N.neg[0] = (double)g.negX; N.neg[1] = (double)g.negY; N.neg[2] = (double)g.negZ;
+    N.corner[0] = (double)__fmul_rn((float)gx, g.cellSize);
+    N.corner[1] = (double)__fmul_rn((float)gy, g.cellSize);
+    N.corner[2] = (double)__fmul_rn((float)gz, g.cellSize);
+    N.scw = ref_scw(g);
+    N.R = 2.0 * N.scw;
+    N.lo = N.R * N.R * (1.0 - 0x1p-48);
+    N.hi = N.R * N.R * (1.0 + 0x1p-48);
+    return N;
+}
+// ref_local with the node's part taken once
+__device__ __forceinline__ double ref_node_local(const RefNode& N, int a, double p) {
+    return ((p - N.neg[a]) - N.corner[a]) + 2.0 * N.scw;
+}
+
+// ORs the voxels of particles i0, i0 + step, ... below `last` (each lane its
+// own range and node) into the lane's words planes[z * kVoxStride + lane].  The
+// whole warp calls; a particle that ref_marks leaves open is tested by all of
+// its lanes, two of the 64 points each.
+constexpr int kVoxStride = 33;  // words of eight planes, plane-major: lane l's plane z at z * 33 + l
+__device__ __forceinline__ void ref_mark_particles(const RefNode& N, uint32_t i0, uint32_t last, uint32_t step,
+                                                   const double* __restrict__ px, const double* __restrict__ py,
+                                                   const double* __restrict__ pz, unsigned long long* planes) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i = i0; __any_sync(0xffffffffu, i < last); i += step) {
+        double lx = 0.0, ly = 0.0, lz = 0.0;
+        uint32_t sx = 0, sy = 0, sz = 0;
+        bool open = false;
+        if (i < last) {
+            lx = ref_node_local(N, 0, px[i]);
+            ly = ref_node_local(N, 1, py[i]);
+            lz = ref_node_local(N, 2, pz[i]);
+            const double qx = lx / N.scw, qy = ly / N.scw, qz = lz / N.scw;
+            sx = sat_u32_d(floor(qx));
+            sy = sat_u32_d(floor(qy));
+            sz = sat_u32_d(floor(qz));
+            unsigned long long plane[3];
+            if (ref_marks(qx, qy, qz, sx, sy, sz, plane)) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) planes[(sz - 1u + (uint32_t)k) * kVoxStride + lane] |= plane[k];
+            } else {
+                // The reference's loops run x from sx - 2 while (unsigned) x < sx + 2,
+                // so a stencil coordinate below 2 on any axis leaves a particle
+                // without marks, and points outside the 8^3 tile never mark.
+                open = !(sx < 2u || sy < 2u || sz < 2u);
+            }
+        }
+        const double hs = N.scw / 2.0;
+        for (uint32_t rest = __ballot_sync(0xffffffffu, open); rest; rest &= rest - 1u) {
+            const int j = __ffs(rest) - 1;
+            const double ax = __shfl_sync(0xffffffffu, lx, j), ay = __shfl_sync(0xffffffffu, ly, j), az = __shfl_sync(0xffffffffu, lz, j);
+            const uint32_t tx = __shfl_sync(0xffffffffu, sx, j), ty = __shfl_sync(0xffffffffu, sy, j), tz = __shfl_sync(0xffffffffu, sz, j);
+#pragma unroll
+            for (uint32_t c = lane; c < 64u; c += 32u) {
+                const int vx = (int)(tx - 2u) + (int)(c >> 4), vy = (int)(ty - 2u) + (int)((c >> 2) & 3u),
+                          vz = (int)(tz - 2u) + (int)(c & 3u);
+                if ((uint32_t)vx >= 8u || (uint32_t)vy >= 8u || (uint32_t)vz >= 8u) continue;
+                const double dx = ax - vx * N.scw, dy = ay - vy * N.scw, dz = az - vz * N.scw;
+                if (ref_within(dx, dy + hs, dz + hs, N.R, N.lo, N.hi) || ref_within(dx + hs, dy, dz + hs, N.R, N.lo, N.hi) ||
+                    ref_within(dx + hs, dy + hs, dz, N.R, N.lo, N.hi))
+                    atomicOr(&planes[vz * kVoxStride + j], 1ull << (vx + 8 * vy));
+            }
+        }
+        __syncwarp();
+    }
+}
+// ref_tile_solid over a tile: a voxel (x, y, z) is solid when bit x of `row`
+// or bit z of `planes` is set (Q3: the y test reads the x index)
+struct RefSolid {
+    uint32_t row, planes;
+    __device__ __forceinline__ unsigned long long plane(uint32_t z) const {
+        return (planes >> z) & 1u ? ~0ull : (unsigned long long)row * 0x0101010101010101ull;
+    }
+    __device__ __forceinline__ uint32_t at(uint32_t id) const { return ((row >> (id & 7u)) | (planes >> (id >> 6))) & 1u; }
+};
+__device__ __forceinline__ RefSolid ref_solid(uint32_t key, const flip_grid& g) {
+    uint32_t gx, gy, gz;
+    ref_decompose(key, g, gx, gy, gz);
+    RefSolid S{0u, 0u};
+    if (ref_tile_clear(gx, gy, gz, g)) return S;
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; ++k) {
+        const uint32_t x = gx * 8u + k, y = gy * 8u + k, z = gz * 8u + k;
+        if (x < 2u || y < 2u || x > (uint64_t)(g.sizeX * 8u) + 2u || y > (uint64_t)(g.sizeY * 8u) + 2u) S.row |= 1u << k;
+        if (z < 2u || z > (uint64_t)(g.sizeZ * 8u) + 2u) S.planes |= 1u << k;
+    }
+    return S;
+}
+
+// getNumberVoxelsUsedPerNode (particles.cu:88-190): mask + count per node,
+// kNodeLanes lanes a node: 32 or 8 take a node's particles in turn, 1 leaves a
+// node to a lane (sparse nodes, whose long ones the whole warp takes first).
+// Every lane gathers in words of its own.  A node of more than `giant`
+// particles (positions clamped to a domain face pile up in its nodes) gets
+// its solid voxels here and the others from ref_voxel_giants_kernel: left to
+// one warp, such nodes were 25 of 38 ms at 64M particles.
 constexpr int kVoxWarps = 8;
+constexpr uint32_t kVoxLong = 8;      // particles above which the warp takes a sparse variant's node together
+constexpr uint32_t kVoxGiant = 1024;  // ... and above which several warps do
+struct VoxWarp {
+    unsigned long long planes[8 * kVoxStride];
+    uint32_t mask[32 * 17];  // rows of 16 words, padded: the masks of the warp's nodes
+};
+template <int kNodeLanes>
 __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_counts_kernel(
     const uint32_t* __restrict__ starts, const uint32_t* __restrict__ keys, uint32_t nodes, uint64_t n,
-    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz, flip_grid g,
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz, flip_grid g, uint32_t giant,
     uint32_t* __restrict__ counts, uint32_t* __restrict__ masks) {
-    __shared__ uint32_t mark[kVoxWarps][16];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t b = blockIdx.x * kVoxWarps + (uint32_t)w;
-    if (b >= nodes) return;  // a whole warp; nothing below synchronises the CTA
-    uint32_t* M = mark[w];
-    // the node's particle range, loaded with the key below
-    const uint32_t first = starts[b], last = (b == nodes - 1) ? (uint32_t)n : starts[b + 1];
-    uint32_t gx, gy, gz;
-    ref_decompose(keys[b], g, gx, gy, gz);  // Q3: particle b's key, not the node's
-    if (ref_tile_clear(gx, gy, gz, g)) {
-        if (lane < 16) M[lane] = 0u;
-    } else {
-#pragma unroll 4
-        for (int q = 0; q < 16; ++q) {
-            const uint32_t bits = __ballot_sync(0xffffffffu, ref_tile_solid((uint32_t)(q * 32 + lane), gx, gy, gz, g));
-            if (lane == 0) M[q] = bits;
-        }
-    }
-    __syncwarp();
-    const double scw = ref_scw(g), hs = scw / 2.0, R = 2.0 * scw;
-    const double R2 = R * R, lo = R2 * (1.0 - 0x1p-48), hi = R2 * (1.0 + 0x1p-48);
-    // up to 32 of the node's particles at a time: lane j loads particle j and
-    // works out its local coordinates (the loads and divisions of all of
-    // them in one round), then the warp walks them in order, each lane
-    // taking two of the 64 points of the particle's stencil
-    for (uint32_t i0 = first; i0 < last; i0 += 32u) {
-        RefLocal Lj{};
-        bool ok = false;
-        if (i0 + (uint32_t)lane < last) {
-            Lj = ref_particle_local(px, py, pz, keys, i0 + (uint32_t)lane, g, scw);
-            ok = !(Lj.sx < 2u || Lj.sy < 2u || Lj.sz < 2u);
-        }
-        for (uint32_t live = __ballot_sync(0xffffffffu, ok); live; live &= live - 1u) {
-            const int j = __ffs(live) - 1;
-            RefLocal L;
-            L.lx = __shfl_sync(0xffffffffu, Lj.lx, j);
-            L.ly = __shfl_sync(0xffffffffu, Lj.ly, j);
-            L.lz = __shfl_sync(0xffffffffu, Lj.lz, j);
-            L.sx = __shfl_sync(0xffffffffu, Lj.sx, j);
-            L.sy = __shfl_sync(0xffffffffu, Lj.sy, j);
-            L.sz = __shfl_sync(0xffffffffu, Lj.sz, j);
+    extern __shared__ __align__(16) unsigned char vox_smem[];
+    VoxWarp& W = reinterpret_cast<VoxWarp*>(vox_smem)[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    constexpr uint32_t kNodes = 32u / kNodeLanes;  // nodes a warp
+    const uint32_t b0 = (blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kNodes;
+    if (b0 >= nodes) return;  // a whole warp; nothing below synchronises the CTA
+    unsigned long long* mine = W.planes + lane;
+    auto clear = [&]() {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int pt = lane + 32 * h;
-                const int x = (int)(L.sx - 2u) + (pt >> 4), y = (int)(L.sy - 2u) + ((pt >> 2) & 3),
-                          z = (int)(L.sz - 2u) + (pt & 3);
-                if ((uint32_t)x >= 8u || (uint32_t)y >= 8u || (uint32_t)z >= 8u) continue;
-                const double dx = L.lx - x * scw, dy = L.ly - y * scw, dz = L.lz - z * scw;
-                if (ref_within(dx, dy + hs, dz + hs, R, lo, hi) || ref_within(dx + hs, dy, dz + hs, R, lo, hi) ||
-                    ref_within(dx + hs, dy + hs, dz, R, lo, hi)) {
-                    const int v = x + y * 8 + z * 64;
-                    atomicOr(&M[v >> 5], 1u << (v & 31));
+        for (int z = 0; z < 8; ++z) mine[z * kVoxStride] = 0ull;
+    };
+    // the node's mask from the 32 lanes' words, into row r
+    auto gather = [&](uint32_t r) {
+        uint32_t word = 0;
+#pragma unroll
+        for (int z = 0; z < 8; ++z) {
+            const unsigned long long v = mine[z * kVoxStride];
+            const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+            if (lane == 2u * z) word = lo;
+            if (lane == 2u * z + 1u) word = hi;
+        }
+        if (lane < 16u) W.mask[17u * r + lane] = word;
+    };
+    const uint32_t r = lane / kNodeLanes, b = b0 + r;  // the lane's node
+    uint32_t first = 0, last = 0;
+    if (b < nodes) {
+        first = starts[b];
+        last = b == nodes - 1u ? (uint32_t)n : starts[b + 1u];
+    }
+    RefNode N = ref_node(b < nodes ? keys[first] : 0u, g);
+    if (last - first > giant) last = first;
+    if (kNodeLanes > 1) {
+        clear();
+        __syncwarp();
+        ref_mark_particles(N, first + lane % kNodeLanes, last, kNodeLanes, px, py, pz, W.planes);
+        if (kNodeLanes == 32) {
+            gather(0);
+        } else {
+#pragma unroll
+            for (int z = 0; z < 8; ++z) {
+                unsigned long long v = mine[z * kVoxStride];
+#pragma unroll
+                for (int o = 1; o < kNodeLanes; o <<= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane % kNodeLanes == 0u) {
+                    W.mask[17u * r + 2u * z] = (uint32_t)v;
+                    W.mask[17u * r + 2u * z + 1u] = (uint32_t)(v >> 32);
                 }
+            }
+        }
+    } else {
+        const bool is_long = last - first > kVoxLong;
+        for (uint32_t rest = __ballot_sync(0xffffffffu, is_long); rest; rest &= rest - 1u) {
+            const int j = __ffs(rest) - 1;
+            const uint32_t f = __shfl_sync(0xffffffffu, first, j), l = __shfl_sync(0xffffffffu, last, j);
+            clear();
+            __syncwarp();
+            ref_mark_particles(ref_node(keys[f], g), f + lane, l, 32u, px, py, pz, W.planes);
+            gather((uint32_t)j);
+        }
+        clear();
+        __syncwarp();
+        ref_mark_particles(N, first, is_long ? first : last, 1u, px, py, pz, W.planes);
+        if (!is_long) {
+#pragma unroll
+            for (int z = 0; z < 8; ++z) {
+                const unsigned long long v = mine[z * kVoxStride];
+                W.mask[17u * lane + 2u * z] = (uint32_t)v;
+                W.mask[17u * lane + 2u * z + 1u] = (uint32_t)(v >> 32);
             }
         }
     }
     __syncwarp();
-    const uint32_t bits = lane < 16 ? M[lane] : 0u;
-    if (lane < 16) masks[(size_t)b * 16 + lane] = bits;
-    uint32_t c = __popc(bits);
+    // solid voxels of tiles on the domain's faces, then the counts
+    if (b < nodes && lane % kNodeLanes == 0u) {
+        uint32_t c = 0;
+        const RefSolid sol = ref_solid(keys[b], g);  // Q3: particle b's key, not the node's
+        if (sol.row | sol.planes)
+            for (uint32_t z = 0; z < 8u; ++z) {
+                const unsigned long long v = sol.plane(z);
+                W.mask[17u * r + 2u * z] |= (uint32_t)v;
+                W.mask[17u * r + 2u * z + 1u] |= (uint32_t)(v >> 32);
+            }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) counts[b] = c;
+        for (int k = 0; k < 16; ++k) c += __popc(W.mask[17u * r + k]);
+        counts[b] = c;
+    }
+    __syncwarp();
+    const uint32_t words = 16u * min(kNodes, nodes - b0);
+    for (uint32_t i = lane; i < words; i += 32u) masks[(size_t)b0 * 16u + i] = W.mask[17u * (i >> 4) + (i & 15u)];
 }
 
-// generateVoxelIDs (particles.cu:192-321): compaction from the mask, a warp
-// per node; lane l writes bit l of each mask word
+// the last node whose first particle is at most p (starts ascend from 0): 32
+// probes a step
+__device__ __forceinline__ uint32_t ref_node_of(const uint32_t* __restrict__ starts, uint32_t nodes, uint32_t p) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0, hi = nodes;
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u, at = lo + lane * step;
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, at < hi && (lane == 0u || starts[at] <= p)));
+        lo += (c - 1u) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+// The nodes of more than kVoxGiant particles: a warp takes kVoxGiant
+// consecutive particles, so a giant node among them holds the first or the
+// last one.  The bits that an atomic OR finds unset are the ones to count.
+__global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_giants_kernel(
+    const uint32_t* __restrict__ starts, const uint32_t* __restrict__ keys, uint32_t nodes, uint64_t n,
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz, flip_grid g,
+    uint32_t* __restrict__ counts, uint32_t* __restrict__ masks) {
+    __shared__ unsigned long long planes[kVoxWarps][8 * kVoxStride];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t p0 = ((uint64_t)blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kVoxGiant;
+    if (p0 >= n) return;  // a whole warp
+    const uint32_t p1 = (uint32_t)min(p0 + kVoxGiant, n);
+    unsigned long long* mine = planes[threadIdx.x >> 5] + lane;
+    uint32_t b = ref_node_of(starts, nodes, (uint32_t)p0);
+    for (int end = 0; end < 2; ++end) {
+        if (end) {
+            const uint32_t e = ref_node_of(starts, nodes, p1 - 1u);
+            if (e == b) return;
+            b = e;
+        }
+        const uint32_t first = starts[b], last = b == nodes - 1u ? (uint32_t)n : starts[b + 1u];
+        if (last - first <= kVoxGiant) continue;
+#pragma unroll
+        for (int z = 0; z < 8; ++z) mine[z * kVoxStride] = 0ull;
+        const RefNode N = ref_node(keys[first], g);
+        const uint32_t i1 = min(last, p1);
+        __syncwarp();
+        ref_mark_particles(N, max(first, (uint32_t)p0) + lane, i1, 32u, px, py, pz, planes[threadIdx.x >> 5]);
+        uint32_t word = 0;
+#pragma unroll
+        for (int z = 0; z < 8; ++z) {
+            const unsigned long long v = mine[z * kVoxStride];
+            const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+            if (lane == 2u * z) word = lo;
+            if (lane == 2u * z + 1u) word = hi;
+        }
+        uint32_t fresh = 0;
+        if (lane < 16u && word) fresh = __popc(word & ~atomicOr(&masks[(size_t)b * 16u + lane], word));
+        fresh = __reduce_add_sync(0xffffffffu, fresh);
+        if (lane == 0u && fresh) atomicAdd(&counts[b], fresh);
+    }
+}
+
+// generateVoxelIDs (particles.cu:192-321): compaction from the masks.  A warp
+// takes 32 nodes: each lane lists its node's voxels into shared memory, and
+// the warp copies the list out in order.  Nodes with more voxels than the list
+// holds, and few nodes (a warp each), are written straight from their masks,
+// lane l the voxel of bit l of each word.
+constexpr uint32_t kIdList = 1280;
+template <int kNodes>
 __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_ids_kernel(
     const uint32_t* __restrict__ keys, uint32_t nodes, const uint32_t* __restrict__ masks,
     const uint32_t* __restrict__ node_voxels, flip_grid g, uint32_t* __restrict__ voxel_ids, int8_t* __restrict__ solids) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t b = blockIdx.x * kVoxWarps + (threadIdx.x >> 5);
-    if (b >= nodes) return;
-    const uint32_t m = lane < 16 ? masks[(size_t)b * 16 + lane] : 0u;
-    // exclusive prefix of the words' popcounts over lanes 0..15
-    uint32_t inc = __popc(m);
+    __shared__ uint16_t lists[kVoxWarps][kNodes > 1 ? kIdList : 1];  // bit 15: solid
+    uint16_t* list = lists[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t b0 = (blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kNodes;
+    if (b0 >= nodes) return;
+    const uint32_t count = min((uint32_t)kNodes, nodes - b0);
+    const uint32_t start = b0 ? node_voxels[b0 - 1u] : 0u, total = node_voxels[b0 + count - 1u] - start;
+    if (kNodes > 1 && total <= kIdList) {
+        if (lane < count) {
+            const uint32_t b = b0 + lane;
+            uint4 m[4];
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+            for (int k = 0; k < 4; ++k) m[k] = reinterpret_cast<const uint4*>(masks + (size_t)b * 16u)[k];
+            uint16_t* at = list + ((lane ? node_voxels[b - 1u] : start) - start);
+            const RefSolid sol = ref_solid(keys[b], g);
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                for (uint32_t word = (&m[k >> 2].x)[k & 3]; word; word &= word - 1u) {
+                    const uint32_t id = 32u * k + (uint32_t)__ffs(word) - 1u;
+                    *at++ = (uint16_t)(id | (sol.at(id) << 15));
+                }
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < total; i += 32u) {
+            const uint32_t v = list[i];
+            voxel_ids[start + i] = v & 511u;
+            solids[start + i] = (int8_t)(v >> 15);
+        }
+        return;
     }
-    const uint32_t pre = inc - __popc(m);
-    uint32_t gx, gy, gz;
-    ref_decompose(keys[b], g, gx, gy, gz);
-    const uint32_t start = b ? node_voxels[b - 1] : 0u;
-    const uint32_t below = (1u << lane) - 1u;
-    const bool clear = ref_tile_clear(gx, gy, gz, g);
-    // the mask words that hold a voxel, in order
-    for (uint32_t rest = __ballot_sync(0xffffffffu, m != 0u); rest; rest &= rest - 1u) {
-        const int q = __ffs(rest) - 1;
-        const uint32_t word = __shfl_sync(0xffffffffu, m, q), base = __shfl_sync(0xffffffffu, pre, q);
-        if ((word >> lane) & 1u) {
-            const uint32_t i = (uint32_t)(q * 32 + lane);
-            const uint32_t pos = start + base + __popc(word & below);
-            voxel_ids[pos] = i;
-            solids[pos] = (!clear && ref_tile_solid(i, gx, gy, gz, g)) ? 1 : 0;
+    for (uint32_t r = 0; r < count; ++r) {
+        const uint32_t b = b0 + r;
+        const uint32_t m = lane < 16u ? masks[(size_t)b * 16u + lane] : 0u;
+        uint32_t at = b ? node_voxels[b - 1u] : 0u;
+        const RefSolid sol = ref_solid(keys[b], g);
+        // the mask words that hold a voxel, in order
+        for (uint32_t rest = __ballot_sync(0xffffffffu, m != 0u); rest; rest &= rest - 1u) {
+            const int q = __ffs(rest) - 1;
+            const uint32_t word = __shfl_sync(0xffffffffu, m, q);
+            if ((word >> lane) & 1u) {
+                const uint32_t i = (uint32_t)q * 32u + lane, pos = at + __popc(word & ((1u << lane) - 1u));
+                voxel_ids[pos] = i;
+                solids[pos] = (int8_t)sol.at(i);
+            }
+            at += __popc(word);
         }
     }
 }
@@ -643,20 +905,38 @@ int ref_launch_ydim(const uint32_t* starts, const uint32_t* keys, uint32_t nodes
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
+// A lane a node where that makes warps for every SM (65,536 nodes: 14 a SM)
+// and a node holds few particles (below 8 a warp's lanes differ little); 8
+// lanes a node for fewer such nodes, a warp a node for dense ones.  The pass
+// over the giants pays its launch from kVoxGiantFrom particles.
+constexpr uint32_t kSparseNodes = 65536;
+constexpr uint64_t kVoxGiantFrom = 32768;
 int ref_launch_voxel_counts(const uint32_t* starts, const uint32_t* keys, uint32_t nodes, uint64_t n, const double* px,
                             const double* py, const double* pz, const flip_grid& g, uint32_t* counts, uint32_t* masks,
                             cudaStream_t s) {
-    if (nodes)
-        ref_voxel_counts_kernel<<<(nodes + kVoxWarps - 1) / kVoxWarps, 32 * kVoxWarps, 0, s>>>(starts, keys, nodes, n, px, py,
-                                                                                            pz, g, counts, masks);
+    if (!nodes) return FLIP_OK;
+    const size_t smem = sizeof(VoxWarp) * kVoxWarps;
+    static_assert(sizeof(VoxWarp) * kVoxWarps <= 49152, "within the default shared memory");
+    const bool giants = n > kVoxGiantFrom;
+    const uint32_t giant = giants ? kVoxGiant : 0xFFFFFFFFu;
+    const int lanes = n < 8ull * nodes ? (nodes >= kSparseNodes ? 1 : 8) : 32;
+    const uint32_t per = 32u / (uint32_t)lanes * kVoxWarps, grid = (nodes + per - 1) / per;
+    const auto kernel = lanes == 1 ? ref_voxel_counts_kernel<1> : (lanes == 8 ? ref_voxel_counts_kernel<8> : ref_voxel_counts_kernel<32>);
+    kernel<<<grid, 32 * kVoxWarps, smem, s>>>(starts, keys, nodes, n, px, py, pz, g, giant, counts, masks);
+    if (giants) {
+        const uint64_t chunk = (uint64_t)kVoxGiant * kVoxWarps;
+        ref_voxel_giants_kernel<<<(unsigned)((n + chunk - 1) / chunk), 32 * kVoxWarps, 0, s>>>(starts, keys, nodes, n, px, py,
+                                                                                           pz, g, counts, masks);
+    }
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
 int ref_launch_voxel_ids(const uint32_t* keys, uint32_t nodes, const uint32_t* masks, const uint32_t* node_voxels,
                          const flip_grid& g, uint32_t* voxel_ids, int8_t* solids, cudaStream_t s) {
-    if (nodes)
-        ref_voxel_ids_kernel<<<(nodes + kVoxWarps - 1) / kVoxWarps, 32 * kVoxWarps, 0, s>>>(keys, nodes, masks, node_voxels, g,
-                                                                                          voxel_ids, solids);
+    if (!nodes) return FLIP_OK;
+    const uint32_t per = (nodes >= kSparseNodes ? 32u : 1u) * kVoxWarps, grid = (nodes + per - 1) / per;
+    const auto kernel = nodes >= kSparseNodes ? ref_voxel_ids_kernel<32> : ref_voxel_ids_kernel<1>;
+    kernel<<<grid, 32 * kVoxWarps, 0, s>>>(keys, nodes, masks, node_voxels, g, voxel_ids, solids);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
