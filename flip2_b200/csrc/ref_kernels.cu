@@ -530,6 +530,39 @@ __device__ __forceinline__ void ref_face_base(int dim, double hs, double& bx, do
     else { by += hs; bx += hs; }
 }
 __device__ __forceinline__ double ref_weight(double d, double R) { return (d > R) ? 0.0 : 1.0 - d / R; }
+// ref_weight of the distance whose square is s, with over2 = 1 / R^2:
+// 1 - sqrt(t), t = s / R^2, 0 from t = 1 on.  The root is Newton's iteration
+// from the FP32 reciprocal root y of t (relative error 2^-22): g = t y, one
+// step g += g (1 - t y^2) / 2 (2^-43), and the remainder t - g^2 added back
+// through y / 2 (below 2^-53), seven multiply-adds against sqrt()'s longer
+// sequence.  A t below 1e-37 counts as such: the weight is 1 either way.
+__device__ __forceinline__ double ref_tent(double s, double over2) {
+    const double t = s * over2;
+    if (t >= 1.0) return 0.0;
+    const float yf = rsqrtf(fmaxf((float)t, 1e-37f));
+    const double y = (double)yf, half = (double)(0.5f * yf);
+    const double g = t * y, e = fma(-g, half, 0.5), g1 = fma(g, e, g);
+    return 1.0 - fma(fma(-g1, g1, t), half, g1);
+}
+
+// one particle's weights and weighted velocities into the node's sums
+__device__ __forceinline__ void ref_scatter(const RefLocal& L, const double (&v)[3], double scw, double hs, double R,
+                                            double (*U)[512], double (*W)[512]) {
+    for (int x = (int)(L.sx - 2u); (uint32_t)x < L.sx + 2u; ++x)
+        for (int y = (int)(L.sy - 2u); (uint32_t)y < L.sy + 2u; ++y)
+            for (int z = (int)(L.sz - 2u); (uint32_t)z < L.sz + 2u; ++z) {
+                if (!((uint32_t)x < 8u && (uint32_t)y < 8u && (uint32_t)z < 8u)) continue;
+                const int id = x + y * 8 + z * 64;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    double bx = x * scw, by = y * scw, bz = z * scw;
+                    ref_face_base(d, hs, bx, by, bz);
+                    double w = ref_weight(ref_dist(L.lx - bx, L.ly - by, L.lz - bz), R);
+                    atomicAdd(&W[d][id], w);
+                    atomicAdd(&U[d][id], __dmul_rn(w, v[d]));
+                }
+            }
+}
 
 // gatherParticleVelsToVoxels for X, Y and Z in one launch (particles.cu:379-488)
 __global__ void __launch_bounds__(kNodeThreads) ref_p2g_kernel(
@@ -555,20 +588,7 @@ __global__ void __launch_bounds__(kNodeThreads) ref_p2g_kernel(
     for (uint32_t idx = starts[b] + threadIdx.x; idx < last; idx += kNodeThreads) {
         RefLocal L = ref_particle_local(px, py, pz, keys, idx, g, scw);
         const double v[3] = {vx[idx], vy[idx], vz[idx]};
-        for (int x = (int)(L.sx - 2u); (uint32_t)x < L.sx + 2u; ++x)
-            for (int y = (int)(L.sy - 2u); (uint32_t)y < L.sy + 2u; ++y)
-                for (int z = (int)(L.sz - 2u); (uint32_t)z < L.sz + 2u; ++z) {
-                    if (!((uint32_t)x < 8u && (uint32_t)y < 8u && (uint32_t)z < 8u)) continue;
-                    const int id = x + y * 8 + z * 64;
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        double bx = x * scw, by = y * scw, bz = z * scw;
-                        ref_face_base(d, hs, bx, by, bz);
-                        double w = ref_weight(ref_dist(L.lx - bx, L.ly - by, L.lz - bz), R);
-                        atomicAdd(&W[d][id], w);
-                        atomicAdd(&U[d][id], __dmul_rn(w, v[d]));
-                    }
-                }
+        ref_scatter(L, v, scw, hs, R, U, W);
     }
     __syncthreads();
     for (uint32_t k = vs + threadIdx.x; k < ve; k += kNodeThreads) {
@@ -580,7 +600,152 @@ __global__ void __launch_bounds__(kNodeThreads) ref_p2g_kernel(
     }
 }
 
-// gatherVoxelVelsToParticles for X, Y and Z (particles.cu:562-662)
+// The same for dense nodes, without atomics: a thread owns one of the 4^3
+// voxel cells a node's particles lie in and one velocity component.  The
+// particles come into shared memory sorted by cell, 512 at a time, and the
+// threads go through the stencil's offsets together, one offset a phase: in
+// a phase no two threads of a component touch one voxel, so each adds its
+// cell's sums with plain additions.  Offsets that no particle of the cell can
+// reach are left out (k = -2 on the component's own axis is two voxels or
+// more away, k = -2 on both others 2.1).  Particles outside those cells (on an
+// upper face, or outside the box) go through the atomics of the other form.
+// FP64 atomics in shared memory are compare-and-swap loops: 1,060 us for
+// 524,264 particles in 1,665 nodes, 478 us this way (what bounds it now: the
+// instructions around a weight, at 18 of 32 lanes, cells holding 8 +- 3).
+constexpr int kP2gThreads = 192;  // three components x 64 cells
+constexpr int kP2gRound = 512;
+struct RefP2gSmem {
+    double U[3][512], W[3][512];
+    double l[3][kP2gRound], v[3][kP2gRound];  // sorted by cell
+    uint32_t count[64], first[65];
+    uint16_t odd[kP2gRound];
+    uint32_t n_odd;
+    int8_t S[512];
+};
+__global__ void __launch_bounds__(kP2gThreads, 4) ref_p2g_cells_kernel(
+    const uint32_t* __restrict__ starts, const uint32_t* __restrict__ keys, uint32_t nodes, uint64_t n,
+    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+    const double* __restrict__ vx, const double* __restrict__ vy, const double* __restrict__ vz,
+    const uint32_t* __restrict__ node_voxels, const uint32_t* __restrict__ voxel_ids, const int8_t* __restrict__ solids,
+    flip_grid g, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
+    extern __shared__ __align__(16) unsigned char p2g_smem[];
+    RefP2gSmem& M = *reinterpret_cast<RefP2gSmem*>(p2g_smem);
+    const uint32_t b = blockIdx.x, tid = threadIdx.x;
+    for (int i = tid; i < 512; i += kP2gThreads) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) M.U[d][i] = M.W[d][i] = 0.0;
+        M.S[i] = 0;
+    }
+    const uint32_t vs = b ? node_voxels[b - 1] : 0u, ve = node_voxels[b];
+    const uint32_t begin = starts[b], end = (b == nodes - 1) ? (uint32_t)n : starts[b + 1];
+    const RefNode N = ref_node(keys[begin], g);
+    const double scw = N.scw, hs = scw / 2.0, R = N.R, over2 = 1.0 / (R * R);
+    const int comp = (int)(tid >> 6), cell = (int)(tid & 63u), ca = cell & 3, cb = (cell >> 2) & 3, cc = cell >> 4;
+    for (uint32_t r0 = begin; r0 < end; r0 += kP2gRound) {
+        const uint32_t m = min((uint32_t)kP2gRound, end - r0);
+        __syncthreads();
+        if (tid < 64u) M.count[tid] = 0u;
+        if (tid == 0) M.n_odd = 0u;
+        __syncthreads();
+        double l[3][3];
+        uint32_t at[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t q = tid + kP2gThreads * (uint32_t)k;
+            at[k] = 0xFFFFFFFFu;
+            if (q < m) {
+                l[k][0] = ref_node_local(N, 0, px[r0 + q]);
+                l[k][1] = ref_node_local(N, 1, py[r0 + q]);
+                l[k][2] = ref_node_local(N, 2, pz[r0 + q]);
+                // (a velocity that is not finite spoils the whole stencil there, weight 0 or not)
+                const double big = fmax(fabs(vx[r0 + q]), fmax(fabs(vy[r0 + q]), fabs(vz[r0 + q])));
+                const bool finite = big < __longlong_as_double(0x7FF0000000000000ll) && !isnan(vx[r0 + q]) &&
+                                    !isnan(vy[r0 + q]) && !isnan(vz[r0 + q]);
+                const uint32_t x = sat_u32_d(floor(l[k][0] / scw)) - 2u, y = sat_u32_d(floor(l[k][1] / scw)) - 2u,
+                               z = sat_u32_d(floor(l[k][2] / scw)) - 2u;
+                if (finite && x < 4u && y < 4u && z < 4u) {
+                    const uint32_t c = x + 4u * y + 16u * z;
+                    at[k] = c | (atomicAdd(&M.count[c], 1u) << 6);
+                } else {
+                    M.odd[atomicAdd(&M.n_odd, 1u)] = (uint16_t)q;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 32u) {  // exclusive scan of 64 counts
+            const uint32_t c0 = M.count[2u * tid], c1 = M.count[2u * tid + 1u];
+            const uint32_t inc = warp_inclusive_scan(c0 + c1);
+            M.first[2u * tid] = inc - c0 - c1;
+            M.first[2u * tid + 1u] = inc - c1;
+            if (tid == 31u) M.first[64] = inc;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (at[k] != 0xFFFFFFFFu) {
+                const uint32_t j = M.first[at[k] & 63u] + (at[k] >> 6), q = r0 + tid + kP2gThreads * (uint32_t)k;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) M.l[d][j] = l[k][d];
+                M.v[0][j] = vx[q];
+                M.v[1][j] = vy[q];
+                M.v[2][j] = vz[q];
+            }
+        __syncthreads();
+        const uint32_t j0 = M.first[cell], j1 = M.first[cell + 1];
+        const double hx = comp == 0 ? 0.0 : hs, hy = comp == 1 ? 0.0 : hs, hz = comp == 2 ? 0.0 : hs;
+        const double* V = M.v[comp];
+        double *Uc = M.U[comp], *Wc = M.W[comp];
+#pragma unroll 1
+        for (int k = 0; k < 64; ++k) {
+            const int kx = k >> 4, ky = (k >> 2) & 3, kz = k & 3;
+            const int own = comp == 0 ? kx : (comp == 1 ? ky : kz), o1 = comp == 0 ? ky : kx, o2 = comp == 2 ? ky : kz;
+            if (own == 0 || (o1 == 0 && o2 == 0)) continue;  // the same for the component's 64 threads
+            // the reference's loops: x from s - 2, s = c + 2
+            const int x = ca + kx, y = cb + ky, z = cc + kz;
+            const double bx = x * scw + hx, by = y * scw + hy, bz = z * scw + hz;
+            // four particles at a time: their chains of dependent FP64 operations overlap
+            double aw = 0.0, au = 0.0;
+            for (uint32_t j = j0; j < j1; j += 4u) {
+                double w[4];
+#pragma unroll
+                for (uint32_t q = 0; q < 4u; ++q) {
+                    const uint32_t i = min(j + q, j1 - 1u);
+                    const double dx = M.l[0][i] - bx, dy = M.l[1][i] - by, dz = M.l[2][i] - bz;
+                    w[q] = ref_tent(fma(dx, dx, fma(dy, dy, dz * dz)), over2);
+                    if (j + q >= j1) w[q] = 0.0;
+                }
+                aw += (w[0] + w[1]) + (w[2] + w[3]);
+#pragma unroll
+                for (uint32_t q = 0; q < 4u; ++q) au = fma(w[q], V[min(j + q, j1 - 1u)], au);
+            }
+            const int id = x + 8 * y + 64 * z;
+            Wc[id] += aw;
+            Uc[id] += au;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + comp) : "memory");
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < M.n_odd; i += kP2gThreads) {
+            const uint32_t q = r0 + M.odd[i];
+            RefLocal L = ref_particle_local(px, py, pz, keys, q, g, scw);
+            const double v[3] = {vx[q], vy[q], vz[q]};
+            ref_scatter(L, v, scw, hs, R, M.U, M.W);
+        }
+    }
+    __syncthreads();
+    for (uint32_t k = vs + tid; k < ve; k += kP2gThreads) M.S[voxel_ids[k]] = solids[k];
+    __syncthreads();
+    for (uint32_t k = vs + tid; k < ve; k += kP2gThreads) {
+        const uint32_t id = voxel_ids[k];
+        const bool sol = M.S[id] != 0;
+        ux[k] = (sol ? 0.0 : M.U[0][id]) / (M.W[0][id] + 0.0000001);
+        uy[k] = (sol ? 0.0 : M.U[1][id]) / (M.W[1][id] + 0.0000001);
+        uz[k] = (sol ? 0.0 : M.U[2][id]) / (M.W[2][id] + 0.0000001);
+    }
+}
+
+// gatherVoxelVelsToParticles for X, Y and Z (particles.cu:562-662).  FP64
+// issue bound (a root and about 15 multiply-adds a weight); the stencil column
+// k = -2 on a component's own axis weighs nothing and is left out.
 __global__ void __launch_bounds__(kNodeThreads) ref_g2p_kernel(
     const uint32_t* __restrict__ starts, const uint32_t* __restrict__ keys, uint32_t nodes, uint64_t n,
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
@@ -599,27 +764,47 @@ __global__ void __launch_bounds__(kNodeThreads) ref_g2p_kernel(
         U[2][id] = uz[k];
     }
     __syncthreads();
-    const uint32_t last = (b == nodes - 1) ? (uint32_t)n : starts[b + 1];
-    const double scw = ref_scw(g), hs = scw / 2.0, R = 2.0 * scw;
-    for (uint32_t idx = starts[b] + threadIdx.x; idx < last; idx += kNodeThreads) {
-        RefLocal L = ref_particle_local(px, py, pz, keys, idx, g, scw);
+    const uint32_t first = starts[b], last = (b == nodes - 1) ? (uint32_t)n : starts[b + 1];
+    const RefNode N = ref_node(keys[first], g);
+    const double scw = N.scw, hs = scw / 2.0, R = N.R, over2 = 1.0 / (R * R);
+    for (uint32_t idx = first + threadIdx.x; idx < last; idx += kNodeThreads) {
+        const double lx = ref_node_local(N, 0, px[idx]), ly = ref_node_local(N, 1, py[idx]), lz = ref_node_local(N, 2, pz[idx]);
+        const uint32_t sx = sat_u32_d(floor(lx / scw)), sy = sat_u32_d(floor(ly / scw)), sz = sat_u32_d(floor(lz / scw));
         double vel[3] = {0.0, 0.0, 0.0}, ws[3] = {0.0, 0.0, 0.0};
-        for (int x = (int)(L.sx - 2u); (uint32_t)x < 8u && (uint32_t)x < L.sx + 2u; ++x)
-            for (int y = (int)(L.sy - 2u); (uint32_t)y < 8u && (uint32_t)y < L.sy + 2u; ++y)
-                for (int z = (int)(L.sz - 2u); (uint32_t)z < 8u && (uint32_t)z < L.sz + 2u; ++z) {
-                    const int id = x + y * 8 + z * 64;
+        // the reference's loops end at the tile's upper edge and do not begin
+        // below its lower one
+        const bool any = sx - 2u < 8u && sy - 2u < 8u && sz - 2u < 8u;
+#pragma unroll 1
+        for (int kx = 0; any && kx < 4; ++kx) {
+            const uint32_t x = sx - 2u + (uint32_t)kx;
+            if (x >= 8u) break;
+            const double dx = lx - (int)x * scw, ex = lx - ((int)x * scw + hs);
+#pragma unroll 1
+            for (int ky = 0; ky < 4; ++ky) {
+                const uint32_t y = sy - 2u + (uint32_t)ky;
+                if (y >= 8u) break;
+                const double dy = ly - (int)y * scw, ey = ly - ((int)y * scw + hs);
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        double bx = x * scw, by = y * scw, bz = z * scw;
-                        ref_face_base(d, hs, bx, by, bz);
-                        double w = ref_weight(ref_dist(L.lx - bx, L.ly - by, L.lz - bz), R);
-                        double u = U[d][id];
+                for (int kz = 0; kz < 4; ++kz) {
+                    const uint32_t z = sz - 2u + (uint32_t)kz;
+                    if (z >= 8u) break;
+                    const double dz = lz - (int)z * scw, ez = lz - ((int)z * scw + hs);
+                    const double ez2 = ez * ez;
+                    const int id = (int)(x + 8u * y + 64u * z);
+                    auto take = [&](int d, bool skip, double s) {
+                        const double u = U[d][id];
+                        const double w = skip ? 0.0 : ref_tent(s, over2);
                         if (u != 0.0) {  // Q10
                             ws[d] += w;
                             vel[d] = fma(w, u, vel[d]);
                         }
-                    }
+                    };
+                    take(0, kx == 0, fma(dx, dx, fma(ey, ey, ez2)));
+                    take(1, ky == 0, fma(ex, ex, fma(dy, dy, ez2)));
+                    take(2, kz == 0, fma(ex, ex, fma(ey, ey, dz * dz)));
                 }
+            }
+        }
         vx[idx] = vel[0] / (ws[0] + 0.00000001);
         vy[idx] = vel[1] / (ws[1] + 0.00000001);
         vz[idx] = vel[2] / (ws[2] + 0.00000001);
@@ -940,13 +1125,22 @@ int ref_launch_voxel_ids(const uint32_t* keys, uint32_t nodes, const uint32_t* m
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
+// cells from this many particles a node on average
+constexpr uint64_t kP2gDense = 32;
 int ref_launch_p2g(const uint32_t* starts, const uint32_t* keys, uint32_t nodes, uint64_t n, const double* px,
                    const double* py, const double* pz, const double* vx, const double* vy, const double* vz,
                    const uint32_t* node_voxels, const uint32_t* voxel_ids, const int8_t* solids, const flip_grid& g,
                    double* ux, double* uy, double* uz, cudaStream_t s) {
-    if (nodes)
+    if (!nodes) return FLIP_OK;
+    if (n >= kP2gDense * nodes) {
+        FLIP_CUDA_TRY(cudaFuncSetAttribute(ref_p2g_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(RefP2gSmem)));
+        ref_p2g_cells_kernel<<<nodes, kP2gThreads, sizeof(RefP2gSmem), s>>>(starts, keys, nodes, n, px, py, pz, vx, vy, vz,
+                                                                           node_voxels, voxel_ids, solids, g, ux, uy, uz);
+    } else {
         ref_p2g_kernel<<<nodes, kNodeThreads, 0, s>>>(starts, keys, nodes, n, px, py, pz, vx, vy, vz, node_voxels, voxel_ids,
                                                       solids, g, ux, uy, uz);
+    }
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
