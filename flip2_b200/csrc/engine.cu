@@ -1066,7 +1066,7 @@ constexpr int kMgCoarseCgIters = 64;
 // done); dot_init >= 0: then FCG's dot products (init: beta = 0), fused into
 // level 0's post-smoothing
 static int mg_cycle(flip_engine* e, bool network, const int* halt, int dot_init = -1) {
-    const int grid0 = nat_grid(e, 5);
+    const int grid0 = nat_grid(e, 4);
     // with the network and a level above the coarsest, the last down kernel
     // also takes the network's input scale
     const bool fused_scale = network && e->mg.levels >= 2;
@@ -2408,6 +2408,9 @@ extern "C" int flip_mg_apply(flip_engine* e, const float* r_lin, float* z_lin) {
     e->warm_ok = false;
     E_CUDA(cudaMemcpyAsync(e->pcg.p0, r_lin, 4 * e->nslots, cudaMemcpyHostToDevice, e->stream));
     E_TRY(nat_launch_lin_tiles_f32(e->pcg.p0, e->pcg.r, e->D, 1, e->stream));
+    // the cycle writes the tiles with fluid cells; the others may hold an
+    // earlier problem's z
+    E_CUDA(cudaMemsetAsync(e->pcg.z, 0, 4 * e->nslots, e->stream));
     E_TRY(mg_setup_problem(e, network));
     E_TRY(mg_cycle(e, network, nullptr));
     E_TRY(nat_launch_lin_tiles_f32(e->pcg.z, e->pcg.p0, e->D, 0, e->stream));
@@ -2437,7 +2440,7 @@ extern "C" int flip_mg_train_step(flip_engine* e, int sample, float lr, double* 
         // the coarsest right-hand side that one V-cycle makes of the residual
         // after k Jacobi-PCG iterations, and its coarse solution (one-CTA CG)
         for (int k = 0; k < sample; ++k) E_TRY(nat_launch_pcg_iteration(e->node_keys, e->d_counts, e->D, e->pcg, e->stream));
-        E_TRY(mg_down(e->mg, nullptr, nat_grid(e, 5), e->stream));
+        E_TRY(mg_down(e->mg, nullptr, nat_grid(e, 4), e->stream));
         E_TRY(mg_cg(c, c.r, e->mg_ev, e->mg_s[0], e->mg_s[1], e->mg_s[2], 1e-6, 4000, e->mg_iters, e->stream));
         e->launches += 2u * (uint32_t)sample + (uint32_t)(e->mg.levels - 1) + 1u;
     } else {

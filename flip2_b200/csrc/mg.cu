@@ -97,20 +97,33 @@ __global__ void __launch_bounds__(512) mg_codes_kernel(MgLevel C, const int* hal
 // box of its tile and a 2-cell halo in shared memory: 16 cells wide in x
 // (x = -4 .. 11, so that every row is four 16-byte quads of the tile
 // layout: x 4..7 of the left tile, the tile's two quads, x 0..3 of the right
-// tile) and 12 in y and z (-2 .. 9).  The first sweep is evaluated on whole
-// quads of the rows y, z = -1 .. 8 (only x = -1 .. 8 of them is used), the
-// second sweep (or the residual) on the tile's 128 quads.  A thread handles
-// four cells: float4 global loads and stores, float4 shared rows.  Vectors
-// are zero off the fluid cells, so a neighbour sum needs no tests; 1/d comes
-// from a shared table.  Five CTAs per SM keep tiles in flight: one CTA's
-// loads overlap the others' barriers and arithmetic.
+// tile) and 12 in y and z (-2 .. 9).  The first sweep is evaluated where the
+// second one (or the residual) reads it: the tile's 64 rows and the 32 rows
+// of its y and z faces, two quads each (a thread a quad), and the cells
+// x = -1 and x = 8 of the tile's rows.  The staged quads are those that this
+// takes: 456 of the box's 576.
+// Vectors are zero off the fluid cells, so a neighbour sum needs no tests.
+// The sweeps work on v = D^-1 r, so that a cell costs its neighbours' sum and
+// two or three multiply-adds; four fluid cells with six non-solid neighbours
+// (nearly all) take 1/6 as a constant, the others 1/d from a shared table.
+// Rows lie 24 floats apart: the 16-byte accesses of a quarter warp, two quads
+// in each of four consecutive rows, then fall on distinct banks (16 apart, two
+// of the rows share theirs, and the shared memory's bandwidth bounds the
+// sweeps).
+// These kernels are bound by instructions and shared memory, not by HBM (6% of
+// its rate): staging all 576 quads with a code test per cell and sweeping all
+// 400 quads of the 10 x 10 rows took 22 and 25 us (down, up) on 2,752 tiles,
+// this 17 and 22 us.  Registers for a fifth CTA per SM cost more (10.9 against
+// 10.5 ms for a step on 16,000 tiles), and so did holding the next tile's loads
+// in registers while one is worked on (10.8 ms).
 constexpr int kMgThreads = 256;
-constexpr int kBX = 16, kBY = 12, kBZ = 12;
-constexpr int kBoxQ = kBX * kBY * kBZ / 4;      // 576 quads in the box
-constexpr int kBoxF = kBX * kBY * kBZ;          // 2304 cells
-constexpr int kSw1Q = 4 * 10 * 10;              // 400 quads of the first sweep
-constexpr int kT1F = kBX * 10 * 10;             // its output box, 1600 cells
-constexpr int kQPer = (kBoxQ + kMgThreads - 1) / kMgThreads;  // 3
+constexpr int kMgCtas = 4;                      // per SM (64 registers a thread)
+constexpr int kBX = 24, kBY = 12, kBZ = 12;      // rows of 16 cells, padded: see above
+constexpr int kBoxF = kBX * kBY * kBZ;
+constexpr int kT1F = kBX * 10 * 10;             // the first sweep's box
+constexpr int kStaged = 456;                    // quads staged
+constexpr int kQPer = (kStaged + kMgThreads - 1) / kMgThreads;  // 2
+constexpr uint32_t kAllSix = 0x86868686u;       // four fluid cells, diagonal 6
 
 // Two FP64 sums over the grid of a level kernel: per-CTA sums into
 // partials[q * gridDim.x + CTA], then the last CTA to arrive adds the
@@ -142,69 +155,136 @@ __device__ __forceinline__ bool mg_last_cta_sum2(double v0, double v1, double* p
     return true;
 }
 
-// box quad q -> (neighbour tile offset + 1 per axis, local slot of its first
-// cell), packed as local | (qx + 1) << 9 | (qy + 1) << 11 | (qz + 1) << 13; -1 past the box
-__device__ __forceinline__ int mg_quad_map(int q) {
-    if (q >= kBoxQ) return -1;
-    const int seg = q & 3, row = q >> 2;
-    const int y = row % kBY - 2, z = row / kBY - 2;
-    const int qx = seg == 0 ? -1 : (seg == 3 ? 1 : 0);
-    const int lx = seg == 0 ? 4 : (seg == 3 ? 0 : 4 * (seg - 1));
-    const int qy = (y + 8) / 8 - 1, qz = (z + 8) / 8 - 1;
-    const int local = lx | ((y - 8 * qy) << 3) | ((z - 8 * qz) << 6);
-    return local | ((qx + 1) << 9) | ((qy + 1) << 11) | ((qz + 1) << 13);
-}
-// slot of a mapped quad's first cell around the tile at tile coordinates
-// (tx, ty, tz), or UINT32_MAX outside the grid; the cell's (i, j, k) out
-__device__ __forceinline__ uint32_t mg_quad_slot(int map, int tx, int ty, int tz, const NatDims& D, int& i, int& j, int& k) {
-    const int ntx = tx + ((map >> 9) & 3) - 1, nty = ty + ((map >> 11) & 3) - 1, ntz = tz + ((map >> 13) & 3) - 1;
-    i = 8 * ntx + (map & 7);
-    j = 8 * nty + ((map >> 3) & 7);
-    k = 8 * ntz + ((map >> 6) & 7);
-    if (map < 0 || ntx < 0 || nty < 0 || ntz < 0 || ntx >= D.tx || nty >= D.ty || ntz >= D.tz) return 0xFFFFFFFFu;
-    return ((uint32_t)(ntx + D.tx * (nty + D.ty * ntz)) << 9) | (uint32_t)(map & 511);
-}
-__device__ __forceinline__ void mg_tile_xyz(uint32_t key, const NatDims& D, int& tx, int& ty, int& tz) {
-    const uint32_t tyz = key / (uint32_t)D.tx;
-    tx = (int)(key - tyz * (uint32_t)D.tx);
-    ty = (int)(tyz % (uint32_t)D.ty);
-    tz = (int)(tyz / (uint32_t)D.ty);
-}
 __device__ __forceinline__ void mg_inv_table(float* inv) {
     if (threadIdx.x < 8) inv[threadIdx.x] = threadIdx.x ? 1.0f / (float)threadIdx.x : 0.0f;
 }
+// row n of the 96 rows of the tile and its y and z faces: (y, z), one of them
+// in 0 .. 7
+__device__ __forceinline__ void mg_face_row(int n, int& y, int& z) {
+    if (n < 64) { y = n & 7; z = n >> 3; }
+    else if (n < 80) { y = n < 72 ? -1 : 8; z = n & 7; }
+    else { y = n & 7; z = n < 88 ? -1 : 8; }
+}
+// A staged quad, as constants of the thread: where it lies in the box and,
+// relative to the tile's first slot, in the grid.
+struct MgQuad {
+    int box;       // float index in the box, -1: none
+    int local;     // slot within its tile
+    int dx, dy, dz;  // the tile it lies in, relative to the CTA's
+    int delta;     // slots from the tile's first slot to the quad's
+};
+__device__ __forceinline__ MgQuad mg_quad(int n, const NatDims& D) {
+    MgQuad Q;
+    Q.box = -1;
+    Q.local = Q.dx = Q.dy = Q.dz = Q.delta = 0;
+    if (n >= kStaged) return Q;
+    int seg, y, z;
+    if (n < 192) {  // x = -2, -1 and x = 8, 9: rows of the tile and its faces
+        seg = n & 1 ? 3 : 0;
+        mg_face_row(n >> 1, y, z);
+    } else {        // the tile's own x range: those rows, the next ones out, the edges
+        const int m = n - 192, r = m >> 1;
+        seg = 1 + (m & 1);
+        if (r < 96) mg_face_row(r, y, z);
+        else if (r < 112) { y = r < 104 ? -2 : 9; z = r & 7; }
+        else if (r < 128) { y = r & 7; z = r < 120 ? -2 : 9; }
+        else { y = (r & 1) ? 8 : -1; z = (r & 2) ? 8 : -1; }
+    }
+    const int lx = seg == 0 ? 4 : (seg == 3 ? 0 : 4 * (seg - 1));
+    Q.dx = seg == 0 ? -1 : (seg == 3 ? 1 : 0);
+    Q.dy = y < 0 ? -1 : (y > 7 ? 1 : 0);
+    Q.dz = z < 0 ? -1 : (z > 7 ? 1 : 0);
+    Q.local = lx | ((y - 8 * Q.dy) << 3) | ((z - 8 * Q.dz) << 6);
+    Q.delta = (Q.dx + D.tx * (Q.dy + D.ty * Q.dz)) * 512 + Q.local;
+    Q.box = 4 * seg + kBX * ((y + 2) + kBY * (z + 2));
+    return Q;
+}
+// a tile of the list: its key and its coordinates (inner: no neighbour lies
+// outside the grid)
+struct MgTile {
+    uint32_t key;
+    int tx, ty, tz;
+    bool inner;
+};
+__device__ __forceinline__ MgTile mg_tile(const MgLevel& L, uint32_t n) {
+    MgTile T;
+    T.key = L.tiles[n];
+    const uint32_t row = T.key / (uint32_t)L.D.tx;
+    T.tx = (int)(T.key - row * (uint32_t)L.D.tx);
+    T.tz = (int)(row / (uint32_t)L.D.ty);
+    T.ty = (int)(row - (uint32_t)T.tz * (uint32_t)L.D.ty);
+    T.inner = T.tx > 0 && T.ty > 0 && T.tz > 0 && T.tx < L.D.tx - 1 && T.ty < L.D.ty - 1 && T.tz < L.D.tz - 1;
+    return T;
+}
+// whether the quad lies in the grid, and its first slot
+__device__ __forceinline__ bool mg_quad_in(const MgQuad& Q, const MgTile& T, const NatDims& D) {
+    return Q.box >= 0 && (T.inner || ((unsigned)(T.tx + Q.dx) < (unsigned)D.tx && (unsigned)(T.ty + Q.dy) < (unsigned)D.ty &&
+                                      (unsigned)(T.tz + Q.dz) < (unsigned)D.tz));
+}
+__device__ __forceinline__ uint32_t mg_quad_slot(const MgQuad& Q, const MgTile& T) { return (uint32_t)((int)(T.key << 9) + Q.delta); }
 __device__ __forceinline__ float f4(const float4& v, int m) { return m == 0 ? v.x : (m == 1 ? v.y : (m == 2 ? v.z : v.w)); }
 __device__ __forceinline__ void f4set(float4& v, int m, float x) {
     if (m == 0) v.x = x; else if (m == 1) v.y = x; else if (m == 2) v.z = x; else v.w = x;
 }
-// one damped Jacobi sweep of a quad: out = u + w D^-1 (r - (d u - nb)) on its
-// fluid cells (0 elsewhere); nb: sums of the six neighbours per cell
-__device__ __forceinline__ float4 mg_quad_sweep(uint32_t c4, const float4& u, const float4& r, const float4& nb,
-                                                const float* inv) {
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+// a * x on the fluid cells by D^-1, 0 elsewhere
+__device__ __forceinline__ float4 mg_over_diag(uint32_t c4, const float4& x, float a, const float* inv) {
+    if (c4 == kAllSix) {
+        const float s = a * (1.0f / 6.0f);
+        return make_float4(s * x.x, s * x.y, s * x.z, s * x.w);
+    }
     float4 o;
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         const uint32_t c = (c4 >> (8 * m)) & 0xFFu;
-        const float d = (float)(c & 7u);
-        const float um = f4(u, m);
-        f4set(o, m, (c & kCellFluid) ? um + kMgOmega * inv[c & 7u] * (f4(r, m) - (d * um - f4(nb, m))) : 0.0f);
+        f4set(o, m, (c & kCellFluid) ? a * inv[c & 7u] * f4(x, m) : 0.0f);
     }
     return o;
 }
+// a sweep of a cell, u + w (v - D^-1 A u): with D^-1 A u = u - nb/d this is
+// (1 - w) u + w v + w nb/d; a fluid cell between six solid ones has A = 0 (and
+// v = 0) and keeps its u
+__device__ __forceinline__ float mg_sweep_cell(uint32_t c, float u, float v, float nb, const float* inv) {
+    const uint32_t d = c & 7u;
+    return (c & kCellFluid) ? fmaf(d ? 1.0f - kMgOmega : 1.0f, u, fmaf(kMgOmega, v, kMgOmega * inv[d] * nb)) : 0.0f;
+}
+__device__ __forceinline__ float4 mg_sweep4(uint32_t c4, const float4& u, const float4& v, const float4& nb, const float* inv) {
+    float4 o;
+    if (c4 == kAllSix) {
+        constexpr float a = 1.0f - kMgOmega, b = kMgOmega * (1.0f / 6.0f);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) f4set(o, m, fmaf(a, f4(u, m), fmaf(kMgOmega, f4(v, m), b * f4(nb, m))));
+        return o;
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) f4set(o, m, mg_sweep_cell((c4 >> (8 * m)) & 0xFFu, f4(u, m), f4(v, m), f4(nb, m), inv));
+    return o;
+}
+// x on the fluid cells, 0 elsewhere
+__device__ __forceinline__ float4 mg_fluid(uint32_t c4, const float4& x) {
+    if (c4 == kAllSix) return x;
+    float4 o;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) f4set(o, m, ((c4 >> (8 * m)) & kCellFluid) ? f4(x, m) : 0.0f);
+    return o;
+}
+__device__ __forceinline__ float4 mg_add(const float4& a, const float4& b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ float4 mg_axpy(float a, const float4& x, const float4& y) {
+    return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
+}
 // neighbour sums of the quad at float index b of a box of row stride SY and
-// plane stride SZ (rows of 16 floats), c its own values, l and r the cells
-// left of its first and right of its last.  The x neighbours come from the
-// neighbouring lanes rather than from scalar shared loads, which hit their
-// banks four times over:
-//   mg_quad_nb_row: the four quads of a row sit in four consecutive active
-//     lanes (qd = the quad's place in its row; the first sweep's layout);
-//   mg_quad_nb_pair: quads 1 and 2 of a row sit in lanes 2k, 2k + 1 of a full
-//     warp (the second sweep's layout); the outer neighbour still comes from
-//     shared memory.
+// plane stride SZ, c its own values.  The tile's two quads of a row lie in
+// neighbouring lanes (an even and an odd one) of a fully active warp, so
+// their common x neighbours come by a shuffle; the outer one is read.
 template <int SY, int SZ>
-__device__ __forceinline__ float4 mg_quad_nb_yz(const float* v, int b, const float4& c, float l, float r) {
-    const float4 ym = *reinterpret_cast<const float4*>(v + b - SY), yp = *reinterpret_cast<const float4*>(v + b + SY);
-    const float4 zm = *reinterpret_cast<const float4*>(v + b - SZ), zp = *reinterpret_cast<const float4*>(v + b + SZ);
+__device__ __forceinline__ float4 mg_quad_nb(const float* v, int b, int half, const float4& c) {
+    const float got = __shfl_xor_sync(0xffffffffu, half ? c.x : c.w, 1);
+    const float outer = v[b + (half ? 4 : -1)];
+    const float l = half ? got : outer, r = half ? outer : got;
+    const float4 ym = ld4(v + b - SY), yp = ld4(v + b + SY), zm = ld4(v + b - SZ), zp = ld4(v + b + SZ);
     float4 s;
     s.x = ((l + c.y) + (ym.x + yp.x)) + (zm.x + zp.x);
     s.y = ((c.x + c.z) + (ym.y + yp.y)) + (zm.y + zp.y);
@@ -213,129 +293,160 @@ __device__ __forceinline__ float4 mg_quad_nb_yz(const float* v, int b, const flo
     return s;
 }
 template <int SY, int SZ>
-__device__ __forceinline__ float4 mg_quad_nb_row(const float* v, int b, int qd, const float4& c) {
-    const unsigned m = __activemask();
-    const float l = __shfl_up_sync(m, c.w, 1), r = __shfl_down_sync(m, c.x, 1);
-    return mg_quad_nb_yz<SY, SZ>(v, b, c, qd > 0 ? l : 0.0f, qd < 3 ? r : 0.0f);
+__device__ __forceinline__ float mg_cell_nb(const float* v, int b) {
+    return ((v[b - 1] + v[b + 1]) + (v[b - SY] + v[b + SY])) + (v[b - SZ] + v[b + SZ]);
 }
-template <int SY, int SZ>
-__device__ __forceinline__ float4 mg_quad_nb_pair(const float* v, int b, int half, const float4& c) {
-    const float got = __shfl_xor_sync(0xffffffffu, half ? c.x : c.w, 1);
-    const float outer = v[b + (half ? 4 : -1)];
-    return mg_quad_nb_yz<SY, SZ>(v, b, c, half ? got : outer, half ? outer : got);
+// The first sweep's places, as constants of the thread: threads 0 .. 191 a
+// quad of the 96 rows, threads 192 .. 255 two of the cells x = -1, x = 8.
+struct MgSweep1 {
+    int box, t, half;     // the quad's float index in the box and in the sweep's box
+    int cell[2], tcell[2];
+};
+__device__ __forceinline__ MgSweep1 mg_sweep1(int tid) {
+    MgSweep1 P;
+    int y, z;
+    mg_face_row(tid < 192 ? tid >> 1 : 0, y, z);
+    P.half = tid & 1;
+    P.box = 4 * (1 + P.half) + kBX * ((y + 2) + kBY * (z + 2));
+    P.t = 4 * (1 + P.half) + kBX * ((y + 1) + 10 * (z + 1));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int row = tid & 63, x = k ? 8 : -1;
+        P.cell[k] = (x + 4) + kBX * ((row & 7) + 2 + kBY * ((row >> 3) + 2));
+        P.tcell[k] = (x + 4) + kBX * ((row & 7) + 1 + 10 * ((row >> 3) + 1));
+    }
+    return P;
 }
+// the tile's own quad of threads 0 .. 127
+struct MgOwn {
+    int half, ly, lz, box, t;
+    uint32_t slot;
+};
+__device__ __forceinline__ MgOwn mg_own(int tid) {
+    MgOwn P;
+    const int row = (tid & 127) >> 1;
+    P.half = tid & 1;
+    P.ly = row & 7;
+    P.lz = row >> 3;
+    P.box = 4 * (1 + P.half) + kBX * ((P.ly + 2) + kBY * (P.lz + 2));
+    P.t = 4 * (1 + P.half) + kBX * ((P.ly + 1) + 10 * (P.lz + 1));
+    P.slot = (uint32_t)(4 * P.half + 8 * P.ly + 64 * P.lz);
+    return P;
+}
+__device__ __forceinline__ uint32_t mg_code(const uint32_t* cb, int cell) { return (cb[cell >> 2] >> (8 * (cell & 3))) & 0xFFu; }
 
-// pre-smoothing and restriction of level F into C:
-//   t1 = w D^-1 r, t = t1 + w D^-1 (r - A t1) (kept in F.t),
+// pre-smoothing and restriction of level F into C.  With v = D^-1 r:
+//   t1 = w v, t = t1 + w D^-1 (r - A t1) = (2 w - w^2) v + w^2 D^-1 sum v
+//   (the sum over the neighbours; t is kept in F.t),
 //   C.r[parent] = 1/2 sum over the 8 children of r - A t (fluid parents; the
 //   parents of a tile are all written by it, and parents of tiles off the
 //   list are never fluid)
 template <bool SCALE = false>
-__global__ void __launch_bounds__(kMgThreads, 5) mg_down_kernel(MgLevel F, MgLevel C, const int* halt, MgScale sc) {
-    pdl_wait();
-    if (mg_halted(halt)) return;
+__global__ void __launch_bounds__(kMgThreads, kMgCtas) mg_down_kernel(MgLevel F, MgLevel C, const int* halt, MgScale sc) {
     // SCALE (C the coarsest level): the sum of C.r^2 and the count over the
     // fluid parents this CTA writes, then *sc.inv_s as mg_scale_kernel sets it
     __shared__ double acc[SCALE ? 2 * 64 : 1];
     if (SCALE && threadIdx.x < 64) acc[2 * threadIdx.x] = acc[2 * threadIdx.x + 1] = 0.0;
-    __shared__ uint32_t cb[kBoxQ];                  // four codes per quad
-    __shared__ __align__(16) float rb[kBoxF];
-    __shared__ __align__(16) float ub[kBoxF];       // t1 = w D^-1 r
-    __shared__ __align__(16) float tb[kT1F];        // first sweep
+    __shared__ uint32_t cb[kBoxF / 4];              // four codes per quad
+    __shared__ __align__(16) float vb[kBoxF];       // v = D^-1 r
+    __shared__ __align__(16) float tb[kT1F];        // t
     __shared__ float S[256];                        // x-pair sums of the residual
     __shared__ float inv[8];
     mg_inv_table(inv);
     const int tid = threadIdx.x;
-    int map[kQPer];
+    MgQuad Q[kQPer];
 #pragma unroll
-    for (int m = 0; m < kQPer; ++m) map[m] = mg_quad_map(tid + m * kMgThreads);
+    for (int m = 0; m < kQPer; ++m) Q[m] = mg_quad(tid + m * kMgThreads, F.D);
+    const MgSweep1 P = mg_sweep1(tid);
+    const MgOwn O = mg_own(tid);
+    pdl_wait();
+    if (mg_halted(halt)) return;
     const uint32_t n = *F.d_ntiles;
     uint32_t pc[kQPer];
-    float4 pr[kQPer];
+    float4 pr[kQPer], ro;
+    MgTile T{};
+    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     auto fetch = [&](uint32_t tt) {
-        int tx, ty, tz, i, j, k;
-        mg_tile_xyz(F.tiles[tt], F.D, tx, ty, tz);
+        T = mg_tile(F, tt);
 #pragma unroll
         for (int m = 0; m < kQPer; ++m) {
-            const uint32_t sl = mg_quad_slot(map[m], tx, ty, tz, F.D, i, j, k);
             pc[m] = 0u;
-            pr[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (sl != 0xFFFFFFFFu) {
+            pr[m] = zero4;
+            if (mg_quad_in(Q[m], T, F.D)) {
+                const uint32_t sl = mg_quad_slot(Q[m], T);
                 pc[m] = *reinterpret_cast<const uint32_t*>(F.cell + sl);
-                pr[m] = *reinterpret_cast<const float4*>(F.r + sl);
+                pr[m] = ld4(F.r + sl);
             }
         }
+        if (tid < 128) ro = ld4(F.r + ((T.key << 9) | O.slot));
     };
     __syncthreads();  // the 1/d table
     for (uint32_t tt = blockIdx.x; tt < n; tt += gridDim.x) {
-        const uint32_t key = F.tiles[tt];
         fetch(tt);
+        const uint32_t now = T.key;
+        const int cx = 4 * T.tx, cy = 4 * T.ty, cz = 4 * T.tz;  // the tile's first parent
+        const float4 r = ro;
 #pragma unroll
-        for (int m = 0; m < kQPer; ++m) {
-            const int q = tid + m * kMgThreads;
-            if (q < kBoxQ) {
-                const uint32_t c4 = pc[m];
-                float4 r, u;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t c = (c4 >> (8 * e)) & 0xFFu;
-                    const float rv = (c & kCellFluid) ? f4(pr[m], e) : 0.0f;
-                    f4set(r, e, rv);
-                    f4set(u, e, kMgOmega * inv[c & 7u] * rv);
-                }
-                cb[q] = c4;
-                *reinterpret_cast<float4*>(rb + 4 * q) = r;
-                *reinterpret_cast<float4*>(ub + 4 * q) = u;
+        for (int m = 0; m < kQPer; ++m)
+            if (Q[m].box >= 0) {
+                cb[Q[m].box >> 2] = pc[m];
+                st4(vb + Q[m].box, mg_over_diag(pc[m], pr[m], 1.0f, inv));
             }
-        }
         __syncthreads();
-        for (int w = tid; w < kSw1Q; w += kMgThreads) {
-            const int qd = w & 3, row = w >> 2;
-            const int by = row % 10 + 1, bz = row / 10 + 1;
-            const int b = 4 * qd + kBX * (by + kBY * bz);
-            const float4 uc = *reinterpret_cast<const float4*>(ub + b);
-            const float4 o = mg_quad_sweep(cb[b >> 2], uc, *reinterpret_cast<const float4*>(rb + b),
-                                           mg_quad_nb_row<kBX, kBX * kBY>(ub, b, qd, uc), inv);
-            *reinterpret_cast<float4*>(tb + 4 * qd + kBX * (row % 10 + 10 * (row / 10))) = o;
+        constexpr float kA = 2.0f * kMgOmega - kMgOmega * kMgOmega, kB = kMgOmega * kMgOmega;
+        if (tid < 192) {
+            const uint32_t c4 = cb[P.box >> 2];
+            const float4 v = ld4(vb + P.box);
+            const float4 nb = mg_quad_nb<kBX, kBX * kBY>(vb, P.box, P.half, v);
+            st4(tb + P.t, mg_axpy(kA, v, mg_over_diag(c4, nb, kB, inv)));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t c = mg_code(cb, P.cell[k]);
+                const float b = (c & kCellFluid) ? kB * inv[c & 7u] : 0.0f;
+                tb[P.tcell[k]] = fmaf(kA, vb[P.cell[k]], b * mg_cell_nb<kBX, kBX * kBY>(vb, P.cell[k]));
+            }
         }
         __syncthreads();
         if (tid < 128) {
-            const int half = tid & 1, row = tid >> 1, ly = row & 7, lz = row >> 3;
-            const int qd = 1 + half;
-            const int b = 4 * qd + kBX * ((ly + 2) + kBY * (lz + 2));
-            const int t = 4 * qd + kBX * ((ly + 1) + 10 * (lz + 1));
-            const uint32_t c4 = cb[b >> 2];
-            const float4 tv = *reinterpret_cast<const float4*>(tb + t), r = *reinterpret_cast<const float4*>(rb + b);
-            const float4 nb = mg_quad_nb_pair<kBX, kBX * 10>(tb, t, half, tv);
+            const uint32_t c4 = cb[O.box >> 2];
+            const float4 tv = ld4(tb + O.t);
+            const float4 nb = mg_quad_nb<kBX, kBX * 10>(tb, O.t, O.half, tv);
             float res[4];
+            if (c4 == kAllSix) {
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const uint32_t c = (c4 >> (8 * m)) & 0xFFu;
-                res[m] = (c & kCellFluid) ? f4(r, m) - ((float)(c & 7u) * f4(tv, m) - f4(nb, m)) : 0.0f;
+                for (int m = 0; m < 4; ++m) res[m] = f4(r, m) - (6.0f * f4(tv, m) - f4(nb, m));
+            } else {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const uint32_t c = (c4 >> (8 * m)) & 0xFFu;
+                    res[m] = (c & kCellFluid) ? f4(r, m) - ((float)(c & 7u) * f4(tv, m) - f4(nb, m)) : 0.0f;
+                }
             }
-            *reinterpret_cast<float4*>(F.t + ((key << 9) | (uint32_t)(4 * half + 8 * ly + 64 * lz))) = tv;
-            S[(2 * half) + 4 * (ly + 8 * lz)] = res[0] + res[1];
-            S[(2 * half + 1) + 4 * (ly + 8 * lz)] = res[2] + res[3];
+            st4(F.t + ((now << 9) | O.slot), tv);
+            S[(2 * O.half) + 4 * (O.ly + 8 * O.lz)] = res[0] + res[1];
+            S[(2 * O.half + 1) + 4 * (O.ly + 8 * O.lz)] = res[2] + res[3];
         }
         __syncthreads();
-        if (tid < 64) {  // parent (pi, pj, pk) of the tile's 4^3 parents
-            int tx, ty, tz;
-            mg_tile_xyz(key, F.D, tx, ty, tz);
-            const int pi = tid & 3, pj = (tid >> 2) & 3, pk = tid >> 4;
+        if (tid >= 192) {  // parent (pi, pj, pk) of the tile's 4^3 parents
+            const int q = tid - 192;
+            const int pi = q & 3, pj = (q >> 2) & 3, pk = q >> 4;
             const int s0 = pi + 4 * (2 * pj + 8 * 2 * pk);
             const float sum = (S[s0] + S[s0 + 4]) + (S[s0 + 32] + S[s0 + 36]);
-            const uint32_t p = mg_slot(4 * tx + pi, 4 * ty + pj, 4 * tz + pk, C.D);
+            const uint32_t p = mg_slot(cx + pi, cy + pj, cz + pk, C.D);
             const bool fl = (C.cell[p] & kCellFluid) != 0;
             const float v = fl ? 0.5f * sum : 0.0f;
             C.r[p] = v;
             if (SCALE && fl) {
-                acc[2 * tid] += (double)v * (double)v;
-                acc[2 * tid + 1] += 1.0;
+                acc[2 * q] += (double)v * (double)v;
+                acc[2 * q + 1] += 1.0;
             }
         }
-        __syncthreads();
+        // the next tile's staging writes only vb and cb, which nothing reads
+        // past the barrier above; its S comes two barriers later
     }
     if (SCALE) {
+        __syncthreads();
         double out[2];
         const bool last = mg_last_cta_sum2(tid < 64 ? acc[2 * tid] : 0.0, tid < 64 ? acc[2 * tid + 1] : 0.0,
                                            sc.partials, sc.ticket, out);
@@ -343,20 +454,18 @@ __global__ void __launch_bounds__(kMgThreads, 5) mg_down_kernel(MgLevel F, MgLev
     }
 }
 
-// two damped Jacobi sweeps from a start vector u: t2 = u + w D^-1 (r - A u),
-// L.z = t2 + w D^-1 (r - A t2).  MODE 0: u = L.t + C.z[parent] (prolongation
-// of the coarse correction; post-smoothing); MODE 1: u = zn + D^-1 r (the
-// coarsest level with the network output zn); MODE 2: u = w D^-1 r (the
-// coarsest level without the network); MODE 3: u = zn (the coarsest level
-// after a CG solve into zn).  DOT (MODE 0 on level 0): FCG's dot products
-// of the z it writes (MgDot), reduced by the last CTA.
+// two damped Jacobi sweeps (mg_sweep_cell) from a start vector u, with v = D^-1 r;
+// the second one's result is L.z.  MODE 0: u = L.t + C.z[parent] (prolongation
+// of the coarse correction; post-smoothing; C.z is zero off the coarse fluid
+// cells); MODE 1: u = zn + v (the coarsest level with the network output zn);
+// MODE 2: u = w v (the coarsest level without the network); MODE 3: u = zn
+// (the coarsest level after a CG solve into zn).  DOT (MODE 0 on level 0):
+// FCG's dot products of the z it writes (MgDot), reduced by the last CTA.
 template <int MODE, bool DOT = false>
-__global__ void __launch_bounds__(kMgThreads, 5) mg_sweeps_kernel(MgLevel L, MgLevel C, const float* __restrict__ zn,
-                                                                  const int* halt, MgDot dot) {
-    pdl_wait();
-    if (mg_halted(halt)) return;
-    __shared__ uint32_t cb[kBoxQ];
-    __shared__ __align__(16) float rb[kBoxF];
+__global__ void __launch_bounds__(kMgThreads, kMgCtas) mg_sweeps_kernel(MgLevel L, MgLevel C, const float* __restrict__ zn,
+                                                                        const int* halt, MgDot dot) {
+    __shared__ uint32_t cb[kBoxF / 4];
+    __shared__ __align__(16) float vb[kBoxF];
     __shared__ __align__(16) float ub[kBoxF];
     __shared__ __align__(16) float tb[kT1F];
     __shared__ float inv[8];
@@ -364,102 +473,85 @@ __global__ void __launch_bounds__(kMgThreads, 5) mg_sweeps_kernel(MgLevel L, MgL
     mg_inv_table(inv);
     const int tid = threadIdx.x;
     if (DOT && tid < 128) acc[2 * tid] = acc[2 * tid + 1] = 0.0;
-    int map[kQPer];
+    MgQuad Q[kQPer];
 #pragma unroll
-    for (int m = 0; m < kQPer; ++m) map[m] = mg_quad_map(tid + m * kMgThreads);
+    for (int m = 0; m < kQPer; ++m) Q[m] = mg_quad(tid + m * kMgThreads, L.D);
+    const MgSweep1 P = mg_sweep1(tid);
+    const MgOwn O = mg_own(tid);
+    pdl_wait();
+    if (mg_halted(halt)) return;
     const uint32_t n = *L.d_ntiles;
+    const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     uint32_t pc[kQPer];
+    MgTile T{};
     float4 pr[kQPer], pu[kQPer];
     float2 pe[kQPer];      // MODE 0: the two parents' corrections
-    uint32_t pp[kQPer];    // MODE 0: the two parents' codes
     auto fetch = [&](uint32_t tt) {
-        int tx, ty, tz, i, j, k;
-        mg_tile_xyz(L.tiles[tt], L.D, tx, ty, tz);
+        T = mg_tile(L, tt);
 #pragma unroll
         for (int m = 0; m < kQPer; ++m) {
-            const uint32_t sl = mg_quad_slot(map[m], tx, ty, tz, L.D, i, j, k);
             pc[m] = 0u;
-            pp[m] = 0u;
-            pr[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            pu[m] = pr[m];
+            pr[m] = pu[m] = zero4;
             pe[m] = make_float2(0.0f, 0.0f);
-            if (sl != 0xFFFFFFFFu) {
+            if (mg_quad_in(Q[m], T, L.D)) {
+                const uint32_t sl = mg_quad_slot(Q[m], T);
                 pc[m] = *reinterpret_cast<const uint32_t*>(L.cell + sl);
-                pr[m] = *reinterpret_cast<const float4*>(L.r + sl);
+                pr[m] = ld4(L.r + sl);
                 if (MODE == 0) {
-                    pu[m] = *reinterpret_cast<const float4*>(L.t + sl);
+                    pu[m] = ld4(L.t + sl);
                     // parents of x, x+1 and of x+2, x+3: consecutive coarse cells
-                    const uint32_t ps = mg_slot(i >> 1, j >> 1, k >> 1, C.D);
+                    const int l = Q[m].local;
+                    const uint32_t ps = mg_slot(4 * (T.tx + Q[m].dx) + ((l & 7) >> 1), 4 * (T.ty + Q[m].dy) + ((l >> 4) & 3),
+                                                4 * (T.tz + Q[m].dz) + (l >> 7), C.D);
                     pe[m] = *reinterpret_cast<const float2*>(C.z + ps);
-                    pp[m] = *reinterpret_cast<const uint16_t*>(C.cell + ps);
                 } else if (MODE == 1 || MODE == 3) {
-                    pu[m] = *reinterpret_cast<const float4*>(zn + sl);
+                    pu[m] = ld4(zn + sl);
                 }
             }
         }
     };
     __syncthreads();  // the 1/d table
     for (uint32_t tt = blockIdx.x; tt < n; tt += gridDim.x) {
-        const uint32_t key = L.tiles[tt];
         fetch(tt);
+        const uint32_t now = T.key;
 #pragma unroll
-        for (int m = 0; m < kQPer; ++m) {
-            const int q = tid + m * kMgThreads;
-            if (q < kBoxQ) {
-                const uint32_t c4 = pc[m];
-                float4 r, u;
+        for (int m = 0; m < kQPer; ++m)
+            if (Q[m].box >= 0) {
+                const float4 v = mg_over_diag(pc[m], pr[m], 1.0f, inv);
+                float4 u = pu[m];
+                if (MODE == 0) u = mg_add(u, make_float4(pe[m].x, pe[m].x, pe[m].y, pe[m].y));
+                if (MODE == 1) u = mg_add(u, v);
+                if (MODE == 2) u = make_float4(kMgOmega * v.x, kMgOmega * v.y, kMgOmega * v.z, kMgOmega * v.w);
+                cb[Q[m].box >> 2] = pc[m];
+                st4(vb + Q[m].box, v);
+                st4(ub + Q[m].box, mg_fluid(pc[m], u));
+            }
+        __syncthreads();
+        float4 q4 = zero4, r4 = zero4;
+        if (DOT && tid < 128) {
+            q4 = ld4(dot.q + ((now << 9) | O.slot));
+            r4 = ld4(L.r + ((now << 9) | O.slot));
+        }
+        if (tid < 192) {
+            const uint32_t c4 = cb[P.box >> 2];
+            const float4 u = ld4(ub + P.box), v = ld4(vb + P.box);
+            const float4 nb = mg_quad_nb<kBX, kBX * kBY>(ub, P.box, P.half, u);
+            st4(tb + P.t, mg_sweep4(c4, u, v, nb, inv));
+        } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t c = (c4 >> (8 * e)) & 0xFFu;
-                    const bool fl = (c & kCellFluid) != 0;
-                    const float rv = fl ? f4(pr[m], e) : 0.0f;
-                    float uv = 0.0f;
-                    if (fl) {
-                        if (MODE == 0) {
-                            // a parent that is not fluid may sit in a tile off
-                            // the coarse list (stale z): it contributes nothing
-                            const uint32_t cp = (pp[m] >> (8 * (e >> 1))) & 0xFFu;
-                            uv = f4(pu[m], e) + ((cp & kCellFluid) ? (e < 2 ? pe[m].x : pe[m].y) : 0.0f);
-                        } else if (MODE == 1) {
-                            uv = f4(pu[m], e) + inv[c & 7u] * rv;
-                        } else if (MODE == 3) {
-                            uv = f4(pu[m], e);
-                        } else {
-                            uv = kMgOmega * inv[c & 7u] * rv;
-                        }
-                    }
-                    f4set(r, e, rv);
-                    f4set(u, e, uv);
-                }
-                cb[q] = c4;
-                *reinterpret_cast<float4*>(rb + 4 * q) = r;
-                *reinterpret_cast<float4*>(ub + 4 * q) = u;
+            for (int k = 0; k < 2; ++k) {
+                tb[P.tcell[k]] = mg_sweep_cell(mg_code(cb, P.cell[k]), ub[P.cell[k]], vb[P.cell[k]],
+                                               mg_cell_nb<kBX, kBX * kBY>(ub, P.cell[k]), inv);
             }
         }
         __syncthreads();
-        for (int w = tid; w < kSw1Q; w += kMgThreads) {
-            const int qd = w & 3, row = w >> 2;
-            const int by = row % 10 + 1, bz = row / 10 + 1;
-            const int b = 4 * qd + kBX * (by + kBY * bz);
-            const float4 uc = *reinterpret_cast<const float4*>(ub + b);
-            const float4 o = mg_quad_sweep(cb[b >> 2], uc, *reinterpret_cast<const float4*>(rb + b),
-                                           mg_quad_nb_row<kBX, kBX * kBY>(ub, b, qd, uc), inv);
-            *reinterpret_cast<float4*>(tb + 4 * qd + kBX * (row % 10 + 10 * (row / 10))) = o;
-        }
-        __syncthreads();
         if (tid < 128) {
-            const int half = tid & 1, row = tid >> 1, ly = row & 7, lz = row >> 3;
-            const int qd = 1 + half;
-            const int b = 4 * qd + kBX * ((ly + 2) + kBY * (lz + 2));
-            const int t = 4 * qd + kBX * ((ly + 1) + 10 * (lz + 1));
-            const uint32_t zs = (key << 9) | (uint32_t)(4 * half + 8 * ly + 64 * lz);
-            float4 q4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (DOT) q4 = *reinterpret_cast<const float4*>(dot.q + zs);
-            const uint32_t c4 = cb[b >> 2];
-            const float4 r4 = *reinterpret_cast<const float4*>(rb + b);
-            const float4 tv = *reinterpret_cast<const float4*>(tb + t);
-            const float4 z = mg_quad_sweep(c4, tv, r4, mg_quad_nb_pair<kBX, kBX * 10>(tb, t, half, tv), inv);
-            *reinterpret_cast<float4*>(L.z + zs) = z;
+            const uint32_t zs = (now << 9) | O.slot;
+            const uint32_t c4 = cb[O.box >> 2];
+            const float4 u = ld4(tb + O.t), v = ld4(vb + O.box);
+            const float4 nb = mg_quad_nb<kBX, kBX * 10>(tb, O.t, O.half, u);
+            const float4 z = mg_sweep4(c4, u, v, nb, inv);
+            st4(L.z + zs, z);
             if (DOT) {
                 double rz = 0.0, zq = 0.0;
 #pragma unroll
@@ -472,7 +564,7 @@ __global__ void __launch_bounds__(kMgThreads, 5) mg_sweeps_kernel(MgLevel L, MgL
                 acc[2 * tid + 1] += zq;
             }
         }
-        __syncthreads();
+        __syncthreads();  // vb and cb before the next tile's staging
     }
     if (DOT) {
         double out[2];
@@ -608,11 +700,11 @@ int mg_plan(int nx, int ny, int nz, float h, MgLevel* L, int max_levels) {
     return levels;
 }
 
-// CTAs of the smoothing kernels: five per SM (grid0 on level 0) and no more
+// CTAs of the smoothing kernels: four per SM (grid0 on level 0) and no more
 // than the level has tiles
 static int mg_grid(const MgLevel& L, int grid0, int level) {
     if (level == 0) return grid0;
-    return (int)(L.ntiles < 740u ? L.ntiles : 740u);
+    return (int)(L.ntiles < 592u ? L.ntiles : 592u);
 }
 
 int mg_build(const MgHierarchy& H, const int* halt, cudaStream_t s) {
@@ -621,6 +713,8 @@ int mg_build(const MgHierarchy& H, const int* halt, cudaStream_t s) {
         const int g = (int)(C.ntiles < 1184u ? C.ntiles : 1184u);
         mg_coarsen_kernel<<<g, 512, 0, s>>>(H.L[l - 1], C, halt);
         mg_codes_kernel<<<g, 512, 0, s>>>(C, halt);
+        // tiles off the list are not written: their corrections read as zero
+        FLIP_CUDA_TRY(cudaMemsetAsync(C.z, 0, (size_t)C.ntiles * 512u * sizeof(float), s));
         // the smoothing of an intermediate level walks its tiles with fluid
         // cells (flags in C.active); the coarsest keeps every tile
         if (l + 1 < H.levels) {
@@ -653,7 +747,7 @@ int mg_down(const MgHierarchy& H, const int* halt, int grid0, cudaStream_t s, bo
 int mg_coarsest(const MgHierarchy& H, const float* zn, const int* halt, cudaStream_t s, bool solved) {
     const int c = H.levels - 1;
     const MgLevel& L = H.L[c];
-    const int g = mg_grid(L, 740, c);
+    const int g = mg_grid(L, 592, c);
     const float* z0 = zn;
     const MgDot nd{};
     if (zn && solved) FLIP_CUDA_TRY(pdl_launch(mg_sweeps_kernel<3>, g, kMgThreads, 0, s, L, L, z0, halt, nd));
