@@ -2320,7 +2320,7 @@ static int lp_loss_backward(flip_engine* e, const float* inv_s, bool want_grad, 
     if (want_grad) {
         E_CUDA(cudaMemsetAsync(e->lp.g, 0, sizeof(float) * kLpNumW, e->stream));
         E_TRY(lp_backward_dev(e->lp, G, inv_s, e->pcg.p1, grid, e->stream));
-        e->launches += 14;
+        e->launches += e->lp.tensor_cores ? 16 : 14;
     }
     if (step) {
         E_TRY(lp_adam(e->lp, lr, e->stream));
@@ -2454,7 +2454,7 @@ extern "C" int flip_mg_train_step(flip_engine* e, int sample, float lr, double* 
     E_TRY(lp_loss_grad(G, e->mg_zn, e->mg_ev, e->mg_wbuf, e->mg_gz, e->lp_scalar, grid, e->stream));
     E_CUDA(cudaMemsetAsync(e->lp.g, 0, sizeof(float) * kLpNumW, e->stream));
     E_TRY(lp_backward_dev(e->lp, G, e->mg.inv_s, e->mg_gz, grid, e->stream));
-    e->launches += 1u + 4u + 2u + 14u;
+    e->launches += 1u + 4u + 2u + (e->lp.tensor_cores ? 16u : 14u);
     if (lr > 0.0f) {
         E_TRY(lp_adam(e->lp, lr, e->stream));
         e->launches += 1;

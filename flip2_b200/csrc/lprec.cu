@@ -588,7 +588,7 @@ static int lp_backward_path(LpNet& net, const LpGrid& G, const float* d_inv_s, c
     }
     // layer 0: Gout = gact (wrt act[0]), input = the three channels
     if (net.tensor_cores) {
-        const int rc = lp_in_wgrad_tc(G, net.dil[0], net.gact, d_inv_s, net.g + kLpWOff[0], net.err, net.sms, st);
+        const int rc = lp_in_wgrad_tc(G, net.dil[0], net.gact, d_inv_s, net.gact2, net.g + kLpWOff[0], net.err, net.sms, st);
         if (rc != FLIP_OK) return rc;
     } else {
         lp_wgrad_kernel<0, 3, 16><<<grid, 512, 0, st>>>(G, net.dil[0], net.gact, nullptr, d_inv_s, 1.0f, G.act_tiles,

@@ -91,9 +91,10 @@ int lp_mid_dgrad_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, const flo
 int lp_mid_wgrad_tc(const LpGrid& G, int dil, const float* gout, const __nv_bfloat16* ain, float* dw, int* err, int sms,
                     cudaStream_t st);
 // the weight gradients of the input layer (3 -> 16; its input channels from
-// G.r, G.type and the scale) and of the output layer (16 -> 1; dL/dout =
-// sign * s * gz on the output tiles) on the tensor cores
-int lp_in_wgrad_tc(const LpGrid& G, int dil, const float* gout, const float* d_inv_s, float* dw, int* err, int sms,
+// G.r, G.type and the scale, laid out in rows: scratch of 16 B per slot) and of
+// the output layer (16 -> 1; dL/dout = sign * s * gz on the output tiles) on the
+// tensor cores
+int lp_in_wgrad_tc(const LpGrid& G, int dil, const float* gout, const float* d_inv_s, void* rows, float* dw, int* err, int sms,
                    cudaStream_t st);
 int lp_out_wgrad_tc(const LpGrid& G, int dil, const float* gz, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
                     float* dw, int* err, int sms, cudaStream_t st);

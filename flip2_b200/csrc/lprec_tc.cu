@@ -101,36 +101,90 @@ __device__ __forceinline__ void tile_origin_tc(uint32_t key, const NatDims& D, i
 }
 }  // namespace
 
-// shared-memory footprint of one CTA for dilation DIL
+// 16 bytes from global to shared memory, zeros where !ok (src is not read then)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// first slot of neighbour nb (x, y, z offsets nb % 3 - 1, nb / 3 % 3 - 1,
+// nb / 9 - 1) of tile key, kNoTile outside the grid or where no activations are
+constexpr uint32_t kNoTile = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t tile_neighbour(const LpGrid& G, uint32_t key, int nb) {
+    const int tx = (int)(key % G.D.tx) + nb % 3 - 1, ty = (int)((key / G.D.tx) % G.D.ty) + (nb / 3) % 3 - 1,
+              tz = (int)(key / (G.D.tx * G.D.ty)) + nb / 9 - 1;
+    if ((unsigned)tx >= (unsigned)G.D.tx || (unsigned)ty >= (unsigned)G.D.ty || (unsigned)tz >= (unsigned)G.D.tz) return kNoTile;
+    const uint32_t t = (uint32_t)(tx + G.D.tx * (ty + G.D.ty * tz));
+    return G.tile_active[t] ? t << 9 : kNoTile;
+}
+// cell (px, py, pz) relative to a tile (-8 .. 15 an axis): the neighbour it
+// lies in and its slot there
+__device__ __forceinline__ int rel_neighbour(int px, int py, int pz) {
+    return ((px >> 3) + 1) + 3 * ((py >> 3) + 1) + 9 * ((pz >> 3) + 1);
+}
+__device__ __forceinline__ uint32_t rel_local(int px, int py, int pz) {
+    return (uint32_t)((px & 7) | ((py & 7) << 3) | ((pz & 7) << 6));
+}
+__device__ __forceinline__ uint4 bf16x8(const float4& a, const float4& b) {
+    uint4 o;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+    h[0] = __floats2bfloat162_rn(a.x, a.y);
+    h[1] = __floats2bfloat162_rn(a.z, a.w);
+    h[2] = __floats2bfloat162_rn(b.x, b.y);
+    h[3] = __floats2bfloat162_rn(b.z, b.w);
+    return o;
+}
+
+// shared-memory footprint of one CTA for dilation DIL.  The planes lie 64
+// bytes more than their size apart, so that a voxel's two stores fall on
+// different banks.  The dilation-4 box leaves room for one CTA per SM, which
+// then has twice the threads.
 template <int DIL>
 struct TcSmem {
     static constexpr int B = 8 + 2 * DIL;                 // box edge
-    static constexpr int kPlane = B * B * B * 16;         // bytes of one 8-channel plane
+    static constexpr int kPlane = B * B * B * 16 + 64;    // bytes of one 8-channel plane
     static constexpr int kBox = 2 * kPlane;
     static constexpr int kW = 27 * 512;                   // 27 taps x (16 co x 16 ci) BF16
     static constexpr int kBytes = kBox + kW + 64;
+    static constexpr int kThreads = DIL == 4 ? 512 : 256;
 };
 
-template <int DIL>
-__global__ void __launch_bounds__(kTcThreads) lp_mid_tc_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb,
-                                                               const __nv_bfloat16* __restrict__ in,
-                                                               __nv_bfloat16* __restrict__ out, int* __restrict__ err) {
+// GRAD = false: out = relu(conv(in)).  GRAD = true, the layer's input
+// gradient: gin[v][ci] = relu'(ain[v][ci]) sum_tap sum_co W[tap][ci][co]
+// in[v - dil off(tap)][co] with in = the output gradient (FP32, rounded to BF16
+// in the box) -- the same GEMM with the taps' offsets mirrored and each tap's
+// weights transposed.
+// Bound by the latency of a tile's steps (stage, MMAs, read back): the box's
+// loads are therefore all in flight at once (cp.async; eight float4 a thread
+// for the FP32 box), and a table of the tile's 27 neighbours, made while the
+// previous tile's MMAs run, takes the lookups out of them.  128^3, 4,096 tiles,
+// dilation 2 and 4: forward 118 and 462 -> 100 and 243 us; the input gradient
+// 131 and 305 us, against 583 us with each voxel's 27 neighbours gathered into a
+// K-major A, 128 voxels at a time.
+template <int DIL, bool GRAD>
+__global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
+    lp_mid_tc_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in_,
+                     const __nv_bfloat16* __restrict__ ain, void* __restrict__ out_, int* __restrict__ err) {
     using S = TcSmem<DIL>;
-    constexpr int B = S::B;
+    constexpr int B = S::B, kThr = S::kThreads;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* box = smem;
     unsigned char* wsm = smem + S::kBox;
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::kBox + S::kW);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kBox + S::kW + 16);
     __shared__ int s_abort;
+    __shared__ uint32_t s_nb[2][27];  // this tile's neighbours and the next one's
     if (G.halt && *G.halt) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // weights: global [tap][ci][co] -> per tap [ci/8][co][ci%8] (K-major B: rows = co)
-    for (int e = tid; e < 27 * 256; e += kTcThreads) {
+    // weights: global [tap][ci][co] -> per tap a K-major B: rows = co, K = ci
+    // (GRAD: rows = ci, K = co)
+    for (int e = tid; e < 27 * 256; e += kThr) {
         const int tap = e >> 8, ci = (e >> 4) & 15, co = e & 15;
-        const int off = tap * 512 + (ci >> 3) * 256 + co * 16 + (ci & 7) * 2;
-        *reinterpret_cast<__nv_bfloat16*>(wsm + off) = wb[e];
+        const int row = GRAD ? ci : co, k = GRAD ? co : ci;
+        *reinterpret_cast<__nv_bfloat16*>(wsm + tap * 512 + (k >> 3) * 256 + row * 16 + (k & 7) * 2) = wb[e];
     }
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
@@ -143,34 +197,63 @@ __global__ void __launch_bounds__(kTcThreads) lp_mid_tc_kernel(LpGrid G, const _
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    const uint32_t n = *G.d_nact;
+    if (warp == 1 && lane < 27 && blockIdx.x < n) s_nb[0][lane] = tile_neighbour(G, G.act_tiles[blockIdx.x], lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
     const uint32_t box_s = smem_u32(box), w_s = smem_u32(wsm), mbar_s = smem_u32(mbar);
-    const uint32_t n = *G.d_nact;
     uint32_t phase = 0;
     bool pending_mma = false;
-    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
+    int cur = 0;
+    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x, cur ^= 1) {
         const uint32_t key = G.act_tiles[t];
         int ox, oy, oz;
         tile_origin_tc(key, G.D, ox, oy, oz);
         // 1. input box, two 16-byte chunks per voxel
-        for (int e = tid; e < 2 * B * B * B; e += kTcThreads) {
-            const int c = e & 1, v = e >> 1;
-            const int bx = v % B, by = (v / B) % B, bz = v / (B * B);
-            const int gx = ox - DIL + bx, gy = oy - DIL + by, gz = oz - DIL + bz;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (gx >= 0 && gy >= 0 && gz >= 0 && gx < G.D.nx && gy < G.D.ny && gz < G.D.nz) {
-                const uint32_t tt = (uint32_t)((gx >> 3) + G.D.tx * ((gy >> 3) + G.D.ty * (gz >> 3)));
-                if (G.tile_active[tt]) {
-                    const uint32_t sl = (tt << 9) | (uint32_t)((gx & 7) | ((gy & 7) << 3) | ((gz & 7) << 6));
-                    val = *reinterpret_cast<const uint4*>(in + (size_t)sl * 16 + c * 8);
+        auto source = [&](int e, uint32_t& sl) {  // its voxel's slot; whether there is one
+            const int v = e >> 1;
+            const int px = v % B - DIL, py = (v / B) % B - DIL, pz = v / (B * B) - DIL;
+            const uint32_t base = s_nb[cur][rel_neighbour(px, py, pz)];
+            const bool ok = base != kNoTile && ox + px < G.D.nx && oy + py < G.D.ny && oz + pz < G.D.nz;
+            sl = ok ? base | rel_local(px, py, pz) : 0u;
+            return ok;
+        };
+        constexpr int kItems = 2 * B * B * B;
+        if (GRAD) {
+            const float* in = static_cast<const float*>(in_);
+            for (int e0 = tid; e0 < kItems; e0 += 4 * kThr) {
+                float4 g[4][2];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int e = e0 + m * kThr;
+                    uint32_t sl;
+                    g[m][0] = g[m][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (e < kItems && source(e, sl)) {
+                        const float4* p = reinterpret_cast<const float4*>(in + (size_t)sl * 16 + (e & 1) * 8);
+                        g[m][0] = p[0];
+                        g[m][1] = p[1];
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int e = e0 + m * kThr;
+                    if (e < kItems)
+                        *reinterpret_cast<uint4*>(box + (e & 1) * S::kPlane + (e >> 1) * 16) = bf16x8(g[m][0], g[m][1]);
                 }
             }
-            *reinterpret_cast<uint4*>(box + c * S::kPlane + v * 16) = val;
+        } else {
+            const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(in_);
+            for (int e = tid; e < kItems; e += kThr) {
+                uint32_t sl;
+                const bool ok = source(e, sl);
+                cp_async16(box_s + (uint32_t)((e & 1) * S::kPlane + (e >> 1) * 16), in + (size_t)sl * 16 + (e & 1) * 8, ok);
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
         }
-        // make the generic-proxy writes visible to the tensor core's async proxy
+        // make the writes visible to the tensor core's async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
         __syncthreads();
@@ -178,19 +261,39 @@ __global__ void __launch_bounds__(kTcThreads) lp_mid_tc_kernel(LpGrid G, const _
         // 2. 8 slices x 27 taps of M=64 N=16 K=16
         if (tid == 0) {
             for (int z = 0; z < 8; ++z) {
-                for (int tap = 0; tap < 27; ++tap) {
-                    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                    const int bz = z + DIL + DIL * dz, by0 = DIL + DIL * dy, bx0 = DIL + DIL * dx;
-                    const uint32_t aoff = (uint32_t)(((bz * B + by0) * B + bx0) * 16);
-                    const uint64_t ad = umma_desc(box_s + aoff, S::kPlane, B * 16);
-                    const uint64_t bd = umma_desc(w_s + tap * 512, 256, 128);
-                    mma_f16(tmem + (uint32_t)(z * 16), ad, bd, kInstrDesc, tap > 0 ? 1u : 0u);
+                if (DIL == 4) {
+                    // a descriptor holds its address in units of 16 B, and the
+                    // taps' offsets are constants: an addition each
+                    const uint64_t bd = umma_desc(w_s, 256, 128);
+                    const uint64_t ad = umma_desc(box_s + (uint32_t)(z * B * B * 16), S::kPlane, B * 16);
+#pragma unroll
+                    for (int tap = 0; tap < 27; ++tap) {
+                        const int at = GRAD ? 26 - tap : tap;  // mirrored
+                        const int aoff = ((DIL * (at / 9)) * B + DIL * ((at / 3) % 3)) * B + DIL * (at % 3);
+                        mma_f16(tmem + (uint32_t)(z * 16), ad + (uint64_t)aoff, bd + (uint64_t)(32 * tap), kInstrDesc,
+                                tap > 0 ? 1u : 0u);
+                    }
+                } else {
+                    // three CTAs share an SM's tensor core: issued as fast as
+                    // above, each one's chains into one accumulator hold up the
+                    // others' (202 us at dilation 2, against 100)
+                    for (int tap = 0; tap < 27; ++tap) {
+                        constexpr int kStep = GRAD ? -DIL : DIL;
+                        const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+                        const int bz = z + DIL + kStep * dz, by0 = DIL + kStep * dy, bx0 = DIL + kStep * dx;
+                        const uint32_t aoff = (uint32_t)(((bz * B + by0) * B + bx0) * 16);
+                        const uint64_t ad = umma_desc(box_s + aoff, S::kPlane, B * 16);
+                        const uint64_t bd = umma_desc(w_s + tap * 512, 256, 128);
+                        mma_f16(tmem + (uint32_t)(z * 16), ad, bd, kInstrDesc, tap > 0 ? 1u : 0u);
+                    }
                 }
             }
             mma_commit(mbar_s);
         }
         pending_mma = true;
-        // 3. epilogue: warp w reads sub-partition w % 4 of slices w/4, w/4+2, w/4+4, w/4+6
+        if (warp == 1 && lane < 27 && t + gridDim.x < n)
+            s_nb[cur ^ 1][lane] = tile_neighbour(G, G.act_tiles[t + gridDim.x], lane);
+        // 3. epilogue: warp w reads sub-partition w % 4 of every (warps / 4)-th slice
         const bool ok = mbar_wait(mbar_s, phase);
         if (!ok) {
             if (lane == 0) atomicExch(&s_abort, 1);
@@ -201,23 +304,38 @@ __global__ void __launch_bounds__(kTcThreads) lp_mid_tc_kernel(LpGrid G, const _
         phase ^= 1u;
         tc_fence_after();
         const int q = warp & 3;
-        for (int zz = warp >> 2; zz < 8; zz += 2) {
+        for (int zz = warp >> 2; zz < 8; zz += kThr / 128) {
             float v[16];
             tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(zz * 16), v);
             if (lane < 16) {
                 const int m = lane + 16 * q;  // row of the slice: x = m % 8, y = m / 8
                 const uint32_t sl = (key << 9) | (uint32_t)((m & 7) | ((m >> 3) << 3) | (zz << 6));
-                uint4 o0, o1;
-                __nv_bfloat162* h0 = reinterpret_cast<__nv_bfloat162*>(&o0);
-                __nv_bfloat162* h1 = reinterpret_cast<__nv_bfloat162*>(&o1);
+                if (GRAD) {
+                    const uint4* ap = reinterpret_cast<const uint4*>(ain + (size_t)sl * 16);
+                    const uint4 q0 = ap[0], q1 = ap[1];
+                    const __nv_bfloat16* a0 = reinterpret_cast<const __nv_bfloat16*>(&q0);
+                    const __nv_bfloat16* a1 = reinterpret_cast<const __nv_bfloat16*>(&q1);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    h0[k] = __floats2bfloat162_rn(fmaxf(v[2 * k], 0.0f), fmaxf(v[2 * k + 1], 0.0f));
-                    h1[k] = __floats2bfloat162_rn(fmaxf(v[8 + 2 * k], 0.0f), fmaxf(v[8 + 2 * k + 1], 0.0f));
+                    for (int c = 0; c < 8; ++c) {
+                        v[c] = __bfloat162float(a0[c]) > 0.0f ? v[c] : 0.0f;
+                        v[8 + c] = __bfloat162float(a1[c]) > 0.0f ? v[8 + c] : 0.0f;
+                    }
+                    float4* dst = reinterpret_cast<float4*>(static_cast<float*>(out_) + (size_t)sl * 16);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                } else {
+                    uint4 o0, o1;
+                    __nv_bfloat162* h0 = reinterpret_cast<__nv_bfloat162*>(&o0);
+                    __nv_bfloat162* h1 = reinterpret_cast<__nv_bfloat162*>(&o1);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        h0[k] = __floats2bfloat162_rn(fmaxf(v[2 * k], 0.0f), fmaxf(v[2 * k + 1], 0.0f));
+                        h1[k] = __floats2bfloat162_rn(fmaxf(v[8 + 2 * k], 0.0f), fmaxf(v[8 + 2 * k + 1], 0.0f));
+                    }
+                    uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(out_) + (size_t)sl * 16);
+                    dst[0] = o0;
+                    dst[1] = o1;
                 }
-                uint4* dst = reinterpret_cast<uint4*>(out + (size_t)sl * 16);
-                dst[0] = o0;
-                dst[1] = o1;
             }
         }
         tc_fence_before();
@@ -234,15 +352,16 @@ __global__ void __launch_bounds__(kTcThreads) lp_mid_tc_kernel(LpGrid G, const _
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
 }
 
-template <int DIL>
-static int launch_mid_tc(const LpGrid& G, const __nv_bfloat16* wb, const __nv_bfloat16* in, __nv_bfloat16* out, int* err,
-                         int sms, cudaStream_t st) {
+template <int DIL, bool GRAD>
+static int launch_mid_tc(const LpGrid& G, const __nv_bfloat16* wb, const void* in, const __nv_bfloat16* ain, void* out,
+                         int* err, int sms, cudaStream_t st) {
     using S = TcSmem<DIL>;
+    const auto kernel = lp_mid_tc_kernel<DIL, GRAD>;
     static bool attr_set = false;  // per process; the attribute is per function
     if (!attr_set) {
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(lp_mid_tc_kernel<DIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
+        FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
         // all of the unified L1 as shared memory, so several CTAs fit per SM
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(lp_mid_tc_kernel<DIL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         attr_set = true;
     }
     // CTAs per SM from the shared-memory budget (each CTA also holds 1 KB of
@@ -252,7 +371,7 @@ static int launch_mid_tc(const LpGrid& G, const __nv_bfloat16* wb, const __nv_bf
     FLIP_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     int per_sm = smem_sm / (S::kBytes + 2048);
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
-    lp_mid_tc_kernel<DIL><<<sms * per_sm, kTcThreads, S::kBytes, st>>>(G, wb, in, out, err);
+    kernel<<<sms * per_sm, S::kThreads, S::kBytes, st>>>(G, wb, in, ain, out, err);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
@@ -401,67 +520,36 @@ __global__ void __launch_bounds__(kSmTcThreads) lp_small_mid_tc_kernel(LpGrid G,
 }
 
 // ------------------------------------------------------------ backward
-// The backward pass of the 16 -> 16 layers on the tensor cores: a persistent
-// grid whose CTAs take 128 consecutive voxels of the active list at a time.
-//
-// Input gradient (dgrad): Gin[v][ci] = relu'(Ain[v][ci]) sum_tap sum_co
-// W[tap][ci][co] Gout[v - dil off(tap)][co], the forward GEMM with the taps
-// mirrored and each tap's weights transposed.  The CTA gathers, for each tap,
-// Gout at its voxels' mirrored neighbours (rounded to BF16; zero outside the
-// grid or in an inactive tile) into a K-major A operand of 128 rows, as the
-// small-grid forward does, and one thread issues 27 M=128 x N=16 x K=16 MMAs
-// with B = the tap's W transposed.  Warps 0-3 read the FP32 sums back (row m
-// in TMEM lane m), multiply by relu'(Ain) and store FP32.
+// The input gradient of the 16 -> 16 layers is lp_mid_tc_kernel<DIL, true>.
 //
 // Weight gradient (wgrad), every layer: dW[tap][ci][co] = sum_v In[v + dil
-// off(tap)][ci] Gout[v][co], a GEMM whose reduction runs over the voxels.
-// The CTA gathers the layer's input at each tap's neighbours into
-// A_buf[group][128 v][8 ci] (for a 16-channel input the groups are (tap,
-// ci / 8)), which reads as an MN-major A: rows m = (group, ci % 8), groups of
-// 8 rows 2 KB apart, the voxels along K 16 B apart.  Gout at its own voxels
-// is staged as an MN-major B (voxels along K, co along N), as its BF16
-// rounding and the BF16 rounding of the remainder, so that the products keep
-// about 16 bits of Gout (and of the input layer's r/s, split the same way
-// into two rows).  M=128 accumulators (16 row groups each) collect 8 K-steps
-// of 16 voxels per chunk over all of the CTA's chunks; at the end warps 0-3
-// add them into dW with FP32 atomics.  Waits are bounded as in the forward
-// kernels.
+// off(tap)][ci] Gout[v][co], a GEMM whose reduction runs over the voxels.  A
+// persistent grid, a CTA per SM, takes the listed tiles in turn and stages a
+// tile's input box, as the forward kernel does, in rows of x for each (z, y, 8-channel
+// half), the rows of y and y + dil next to each other.  K = 16 voxels are the
+// rows y and y + dil of a z-slice (8 voxels each, 16 B apart), and M = 64 rows
+// are eight consecutive box rows of 8 channels: the taps dy = -1, 0, 1 of one
+// (dz, dx) with their halves, read straight from the box as an MN-major A,
+// and two more that come to nothing.  So a K-step is nine MMAs, one per (dz,
+// dx), each into its own accumulator.  Gout at the tile's own voxels is an
+// MN-major B (voxels along K, co along N): its BF16 rounding in columns 0-15 and
+// the BF16 rounding of the remainder in columns 16-31, so that the products
+// keep about 16 bits of Gout (and of the input layer's r/s, split the same way
+// into two rows).  The accumulators collect all of a CTA's tiles; at the end
+// warps 0-3 add them into dW with FP32 atomics.
+//
+// What bounds it at dilation 4 is the box's way from L2 (8 times the tile),
+// below that its 288 MMAs a tile, some 65 cycles each.  Up to dilation 2 two
+// boxes fit, and the next tile's copies (cp.async) run beside the MMAs.  128^3,
+// 4,096 tiles: 16 -> 16 layers 275 and 285 us (dilation 2 and 4), 16 -> 1 218 us,
+// 3 -> 16 205 us.  Gathering all 27 neighbours of each voxel into one A operand
+// took 610 us (both dilations), 480 and 560 us with a wait for the MMAs before the
+// next gather, and 460, 420 and 270 us with three stages of copies ahead of
+// them: 27 reads of a voxel from L2 instead of 3.4 or 8.
+// Waits are bounded as in the forward kernels.
 namespace {
-constexpr int kBwThreads = 256;
-constexpr int kBwRows = 128;
-constexpr int kDgA = 27 * kBwRows * 32;  // 27 taps x 128 rows x 16 BF16
-constexpr int kDgBytes = kDgA + 27 * 512 + 64;
-constexpr int kWgB = 2 * 2 * kBwRows * 16;  // B: high and low part x two co halves x 128 rows
-constexpr uint32_t kInstrDescMN = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((16u >> 3) << 17) |
-                                  ((128u >> 4) << 24);  // FP32 += BF16 x BF16, A and B MN-major, N=16, M=128
+constexpr int kBwThreads = 512;
 
-// slot of voxel vx of the active list and its cell (i, j, k)
-__device__ __forceinline__ uint32_t bw_voxel(const LpGrid& G, uint32_t vx, int& i, int& j, int& k) {
-    const uint32_t key = G.act_tiles[vx >> 9];
-    int ox, oy, oz;
-    tile_origin_tc(key, G.D, ox, oy, oz);
-    const int l = (int)(vx & 511u);
-    i = ox + (l & 7);
-    j = oy + ((l >> 3) & 7);
-    k = oz + (l >> 6);
-    return (key << 9) | (uint32_t)l;
-}
-// slot of (i, j, k) if it is in the grid and in an active tile, else UINT32_MAX
-__device__ __forceinline__ uint32_t bw_active(const LpGrid& G, int i, int j, int k) {
-    if (i < 0 || j < 0 || k < 0 || i >= G.D.nx || j >= G.D.ny || k >= G.D.nz) return 0xFFFFFFFFu;
-    const uint32_t t = (uint32_t)((i >> 3) + G.D.tx * ((j >> 3) + G.D.ty * (k >> 3)));
-    if (!G.tile_active[t]) return 0xFFFFFFFFu;
-    return (t << 9) | (uint32_t)((i & 7) | ((j & 7) << 3) | ((k & 7) << 6));
-}
-__device__ __forceinline__ uint4 bf16x8(const float4& a, const float4& b) {
-    uint4 o;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
-    h[0] = __floats2bfloat162_rn(a.x, a.y);
-    h[1] = __floats2bfloat162_rn(a.z, a.w);
-    h[2] = __floats2bfloat162_rn(b.x, b.y);
-    h[3] = __floats2bfloat162_rn(b.z, b.w);
-    return o;
-}
 // the BF16 rounding of what bf16x8 dropped
 __device__ __forceinline__ uint4 bf16x8_rest(const float4& a, const float4& b, const uint4& hi) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&hi);
@@ -470,365 +558,273 @@ __device__ __forceinline__ uint4 bf16x8_rest(const float4& a, const float4& b, c
     return bf16x8(make_float4(a.x - h0.x, a.y - h0.y, a.z - h1.x, a.w - h1.y),
                   make_float4(b.x - h2.x, b.y - h2.y, b.z - h3.x, b.w - h3.y));
 }
-__device__ __forceinline__ void tc_init(uint64_t* mbar, uint32_t* tslot, int* s_abort, uint32_t cols) {
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *s_abort = 0;
-    }
-    if ((threadIdx.x >> 5) == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-}
 }  // namespace
 
-__global__ void __launch_bounds__(kBwThreads) lp_tc_dgrad_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, int dil,
-                                                                 const float* __restrict__ gout,
-                                                                 const __nv_bfloat16* __restrict__ ain,
-                                                                 float* __restrict__ gin, int* __restrict__ err) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* abuf = smem;
-    unsigned char* wsm = smem + kDgA;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kDgA + 27 * 512);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kDgA + 27 * 512 + 16);
-    __shared__ int s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t nvox = *G.d_nact * 512u;
-    if (blockIdx.x * kBwRows >= nvox) return;
-    // weights: global [tap][ci][co] -> per tap [co/8][ci][co%8] (K-major B: rows = ci, K = co)
-    for (int e = tid; e < 27 * 256; e += kBwThreads) {
-        const int tap = e >> 8, ci = (e >> 4) & 15, co = e & 15;
-        *reinterpret_cast<__nv_bfloat16*>(wsm + tap * 512 + (co >> 3) * 256 + ci * 16 + (co & 7) * 2) = wb[e];
-    }
-    tc_init(mbar, tslot, &s_abort, 32);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t a_s = smem_u32(abuf), w_s = smem_u32(wsm), mbar_s = smem_u32(mbar);
-    uint32_t phase = 0;
-    bool pending = false;
-    for (uint32_t v0 = blockIdx.x * kBwRows; v0 < nvox; v0 += gridDim.x * kBwRows) {
-        {  // A: thread (row r, half h) gathers its voxel's 27 mirrored neighbours
-            const int h = tid & 1, r = tid >> 1;
-            const uint32_t vx = v0 + (uint32_t)r;
-            int ci = 0, cj = 0, ck = 0;
-            const bool have = vx < nvox;
-            if (have) bw_voxel(G, vx, ci, cj, ck);
-            unsigned char* dst = abuf + h * (kBwRows * 16) + r * 16;
-#pragma unroll
-            for (int t0 = 0; t0 < 27; t0 += 9) {
-                float4 g0[9], g1[9];
-#pragma unroll
-                for (int jj = 0; jj < 9; ++jj) {
-                    const int tap = t0 + jj;
-                    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                    g0[jj] = g1[jj] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    const uint32_t u = have ? bw_active(G, ci - dil * dx, cj - dil * dy, ck - dil * dz) : 0xFFFFFFFFu;
-                    if (u != 0xFFFFFFFFu) {
-                        const float4* p = reinterpret_cast<const float4*>(gout + (size_t)u * 16 + h * 8);
-                        g0[jj] = p[0];
-                        g1[jj] = p[1];
-                    }
-                }
-#pragma unroll
-                for (int jj = 0; jj < 9; ++jj)
-                    *reinterpret_cast<uint4*>(dst + (t0 + jj) * (kBwRows * 32)) = bf16x8(g0[jj], g1[jj]);
-            }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
-            for (int tap = 0; tap < 27; ++tap) {
-                const uint64_t ad = umma_desc(a_s + (uint32_t)(tap * kBwRows * 32), kBwRows * 16, 128);
-                const uint64_t bd = umma_desc(w_s + (uint32_t)(tap * 512), 256, 128);
-                mma_f16(tmem, ad, bd, kInstrDescM128, tap > 0 ? 1u : 0u);
-            }
-            mma_commit(mbar_s);
-        }
-        pending = true;
-        // one decision for the whole CTA: the TMEM reads below are warp-collective
-        if (!mbar_wait(mbar_s, phase) && lane == 0) atomicExch(&s_abort, 1);
-        __syncthreads();
-        if (s_abort) break;
-        pending = false;
-        phase ^= 1u;
-        tc_fence_after();
-        if (warp < 4) {
-            float acc[16];
-            tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16), acc);
-            const uint32_t vx = v0 + (uint32_t)(32 * warp + lane);
-            if (vx < nvox) {
-                const uint32_t sl = (G.act_tiles[vx >> 9] << 9) | (vx & 511u);
-                const uint4* ap = reinterpret_cast<const uint4*>(ain + (size_t)sl * 16);
-                const uint4 q0 = ap[0], q1 = ap[1];
-                const __nv_bfloat16* a0 = reinterpret_cast<const __nv_bfloat16*>(&q0);
-                const __nv_bfloat16* a1 = reinterpret_cast<const __nv_bfloat16*>(&q1);
-                float o[16];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    o[c] = __bfloat162float(a0[c]) > 0.0f ? acc[c] : 0.0f;
-                    o[8 + c] = __bfloat162float(a1[c]) > 0.0f ? acc[8 + c] : 0.0f;
-                }
-                float4* dp = reinterpret_cast<float4*>(gin + (size_t)sl * 16);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) dp[m] = make_float4(o[4 * m], o[4 * m + 1], o[4 * m + 2], o[4 * m + 3]);
-            }
-        }
-        tc_fence_before();
-        __syncthreads();  // TMEM and the A operand are free for the next chunk
-        tc_fence_after();
-    }
-    if (s_abort) {
-        if (tid == 0) atomicOr(err, 1);
-        if (pending) mbar_wait(mbar_s, phase);  // bounded: the MMAs before TMEM is freed
-        __syncthreads();
-    }
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32) : "memory");
-}
-
-// Weight-gradient layouts per layer (WG): the A row groups of 8 (MN-major,
-// 2 KB apart), the accumulators, and the B parts.
-//   WG 1 (16 -> 16): groups (tap, half) = 54, rows ci % 8; B = Gout [slot][16]
-//                    as a high and a low part (two MMAs per step).
-//   WG 2 (16 -> 1):  groups as WG 1; B = s gz [slot] with its high part in
-//                    column 0 and its low part in column 1 (one MMA per step);
+// Weight-gradient layouts per layer (WG): the box rows, the accumulators'
+// M rows and B's columns.
+//   WG 1 (16 -> 16): two halves a row, M rows (dy, half, ci % 8); B = Gout
+//                    [slot][16] as a high and a low part, N = 32; dW = their sum.
+//   WG 2 (16 -> 1):  rows as WG 1; B = s gz [slot] with its high part in
+//                    column 0 and its low part in column 1, N = 16;
 //                    dW = column 0 + column 1.  Voxels: the output list.
-//   WG 0 (3 -> 16):  groups tap = 27, rows [r/s high, fluid, solid, r/s low,
-//                    0, 0, 0, 0] from the input channels; B as WG 1;
-//                    dW[.][0] = row 0 + row 3.
-template <int WG>
+//   WG 0 (3 -> 16):  one row of [r/s high, fluid, solid, r/s low, 0, 0, 0, 0] as
+//                    lp_in_rows_kernel lays them out, M rows (dy, channel); B as
+//                    WG 1; dW[.][0] = channel 0 + channel 3.
+template <int WG, int DIL>
 struct WgShape {
-    static constexpr int kGroups = WG == 0 ? 32 : 64;  // padded to whole M=128 accumulators
-    static constexpr int kUsed = WG == 0 ? 27 : 54;
-    static constexpr int kAcc = kGroups / 16;
-    static constexpr int kParts = WG == 2 ? 1 : 2;
-    static constexpr int kA = kGroups * kBwRows * 16;
-    static constexpr int kBytes = kA + kWgB + 64;
+    static constexpr int B = 8 + 2 * DIL;
+    static constexpr int kHalves = WG == 0 ? 1 : 2;
+    static constexpr int kRow = B * 16 + (DIL == 4 ? 64 : 0);  // bytes of a box row (a voxel's halves on different banks)
+    static constexpr int kBox = B * B * kHalves * kRow;
+    static constexpr int kN = WG == 2 ? 16 : 32;
+    static constexpr int kPart = 512 * 16;                     // bytes of eight of B's columns
+    // B follows the box: the rows past a block of y that the MMAs read end in it
+    static constexpr int kStage = kBox + (kN / 8) * kPart;
+    static constexpr int kStages = 2 * kStage <= 220 * 1024 ? 2 : 1;
+    static constexpr int kBytes = kStages * kStage + 64;
+    static constexpr uint32_t kCols = WG == 2 ? 256 : 512;     // 9 accumulators of kN columns
+    // FP32 += BF16 x BF16, A and B MN-major, N, M=64
+    static constexpr uint32_t kInstr = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                                       ((uint32_t)(kN >> 3) << 17) | ((64u >> 4) << 24);
+    static_assert(kBytes <= 226 * 1024, "a stage has to fit");
+    // box row of (z, y) in box coordinates
+    __device__ static constexpr int row(int bz, int by) { return (bz * B + (by % DIL) * (B / DIL) + by / DIL) * kHalves; }
 };
 
-template <int WG>
-__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, int dil, const float* __restrict__ gout,
+// the input layer's A rows, 16 bytes per slot of the active tiles
+__global__ void __launch_bounds__(512) lp_in_rows_kernel(LpGrid G, const float* __restrict__ d_inv_s, uint4* __restrict__ rows) {
+    const float inv_s = *d_inv_s;
+    const uint32_t n = *G.d_nact;
+    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
+        const uint32_t u = (G.act_tiles[t] << 9) | threadIdx.x;
+        const uint8_t ty = G.type[u];
+        const float x = (ty == kFluid && G.r) ? G.r[u] * inv_s : 0.0f;
+        const __nv_bfloat16 xh = __float2bfloat16_rn(x);
+        uint4 v;
+        __nv_bfloat162* hv = reinterpret_cast<__nv_bfloat162*>(&v);
+        hv[0] = __halves2bfloat162(xh, __float2bfloat16_rn(ty == kFluid ? 1.0f : 0.0f));
+        hv[1] = __floats2bfloat162_rn(ty == kSolid ? 1.0f : 0.0f, x - __bfloat162float(xh));
+        hv[2] = hv[3] = __floats2bfloat162_rn(0.0f, 0.0f);
+        rows[u] = v;
+    }
+}
+
+template <int WG, int DIL>
+__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const float* __restrict__ gout,
                                                                  const __nv_bfloat16* __restrict__ ain,
                                                                  const float* __restrict__ d_inv_s, float sign,
                                                                  const uint32_t* __restrict__ tiles,
                                                                  const uint32_t* __restrict__ d_n, float* __restrict__ dw,
                                                                  int* __restrict__ err) {
-    using S = WgShape<WG>;
-    extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char* abuf = smem;
-    unsigned char* bbuf = smem + S::kA;  // [part][co half][128 v][8 co]
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::kA + kWgB);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kA + kWgB + 16);
-    __shared__ int s_abort;
+    using S = WgShape<WG, DIL>;
+    constexpr int B = S::B, H = S::kHalves, kStages = S::kStages;
+    extern __shared__ __align__(1024) unsigned char smem[];  // stages of the box, then B: [part][co half][512 v][8 co]
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kStages * S::kStage);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kStages * S::kStage + 32);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t nvox = *d_n * 512u;
-    if (blockIdx.x * kBwRows >= nvox) return;
-    const float inv_s = (WG == 1) ? 1.0f : *d_inv_s;
-    // the row groups past the used ones stay zero, and so do the B columns
-    // that WG 2 leaves empty
-    for (int e = tid; e < (S::kGroups - S::kUsed) * kBwRows; e += kBwThreads)
-        *reinterpret_cast<uint4*>(abuf + S::kUsed * kBwRows * 16 + e * 16) = make_uint4(0u, 0u, 0u, 0u);
-    if (WG == 2)
-        for (int e = tid; e < kWgB / 16; e += kBwThreads) *reinterpret_cast<uint4*>(bbuf + e * 16) = make_uint4(0u, 0u, 0u, 0u);
-    tc_init(mbar, tslot, &s_abort, 64);
+    const uint32_t n = *d_n;
+    if (blockIdx.x >= n) return;
+    const float scale = WG == 2 ? sign / *d_inv_s : 1.0f;
+    if (WG == 2)  // the columns that stay empty
+        for (int e = tid; e < kStages * 2 * 512; e += kBwThreads)
+            *reinterpret_cast<uint4*>(smem + (e >> 10) * S::kStage + S::kBox + (e & 1023) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) {
+        for (int s = 0; s < kStages; ++s)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + s)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(S::kCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const uint32_t a_s = smem_u32(abuf), b_s = smem_u32(bbuf), mbar_s = smem_u32(mbar);
-    uint32_t phase = 0;
-    bool pending = false, any = false;
-    for (uint32_t v0 = blockIdx.x * kBwRows; v0 < nvox; v0 += gridDim.x * kBwRows) {
-        {
-            const int h = tid & 1, r = tid >> 1;
-            const uint32_t vx = v0 + (uint32_t)r;
-            int ci = 0, cj = 0, ck = 0;
-            const bool have = vx < nvox;
-            uint32_t self = 0;
-            if (have) {
-                const uint32_t key = tiles[vx >> 9];
-                int ox, oy, oz;
-                tile_origin_tc(key, G.D, ox, oy, oz);
-                const int l = (int)(vx & 511u);
-                ci = ox + (l & 7);
-                cj = oy + ((l >> 3) & 7);
-                ck = oz + (l >> 6);
-                self = (key << 9) | (uint32_t)l;
-            }
-            // B: the output gradient at the voxel itself
-            if (WG == 2) {
-                if (h == 0) {
-                    const float g = have ? gout[self] * (sign / inv_s) : 0.0f;
-                    const __nv_bfloat16 hi = __float2bfloat16_rn(g);
-                    const __nv_bfloat16 lo = __float2bfloat16_rn(g - __bfloat162float(hi));
-                    __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(bbuf + r * 16);
-                    row[0] = hi;
-                    row[1] = lo;
-                }
-            } else {
-                float4 g0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), g1 = g0;
-                if (have) {
-                    const float4* p = reinterpret_cast<const float4*>(gout + (size_t)self * 16 + h * 8);
-                    g0 = p[0];
-                    g1 = p[1];
-                }
-                const uint4 hi = bf16x8(g0, g1);
-                *reinterpret_cast<uint4*>(bbuf + h * (kBwRows * 16) + r * 16) = hi;
-                *reinterpret_cast<uint4*>(bbuf + 2 * kBwRows * 16 + h * (kBwRows * 16) + r * 16) = bf16x8_rest(g0, g1, hi);
-            }
-            if (WG == 0) {
-                // A: the three input channels at taps 14 h .. 14 h + 13, group = tap
-                for (int tap = 14 * h; tap < 14 * h + 14 && tap < 27; ++tap) {
-                    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                    const uint32_t u = have ? bw_active(G, ci + dil * dx, cj + dil * dy, ck + dil * dz) : 0xFFFFFFFFu;
-                    float x = 0.0f, fl = 0.0f, so = 0.0f;
-                    if (u != 0xFFFFFFFFu) {
-                        const uint8_t t = G.type[u];
-                        fl = t == kFluid ? 1.0f : 0.0f;
-                        so = t == kSolid ? 1.0f : 0.0f;
-                        x = (t == kFluid && G.r) ? G.r[u] * inv_s : 0.0f;
-                    }
-                    const __nv_bfloat16 xh = __float2bfloat16_rn(x);
-                    const float xl = x - __bfloat162float(xh);
-                    uint4 v;
-                    __nv_bfloat162* hv = reinterpret_cast<__nv_bfloat162*>(&v);
-                    hv[0] = __halves2bfloat162(xh, __float2bfloat16_rn(fl));
-                    hv[1] = __floats2bfloat162_rn(so, xl);
-                    hv[2] = hv[3] = __floats2bfloat162_rn(0.0f, 0.0f);
-                    *reinterpret_cast<uint4*>(abuf + tap * (kBwRows * 16) + r * 16) = v;
-                }
-            } else {
-                // A: the activations at the voxel's 27 neighbours, group (tap, h)
-                unsigned char* dst = abuf + h * (kBwRows * 16) + r * 16;
+    const uint32_t smem_s = smem_u32(smem), mbar_s = smem_u32(mbar);
+
+    // lane nb < 27 of every warp holds the first slot of the tile's neighbour
+    // nb (a shuffle looks one up); the next tile's, and the key of the one
+    // after it, are loaded a tile ahead
+    auto key_at = [&](uint32_t t) { return tiles[t < n ? t : n - 1u]; };
+    auto around = [&](uint32_t k) { return lane < 27 ? tile_neighbour(G, k, lane) : kNoTile; };
+    uint32_t key = key_at(blockIdx.x), key1 = key_at(blockIdx.x + gridDim.x), nb = around(key);
+    auto gather = [&](uint32_t t, int stage) {  // the tile key of the list's t-th place; moves on to the next one
+        unsigned char* st = smem + stage * S::kStage;
+        // Gout at the tile's voxels: loads now, stores after the box's copies
+        float4 g[2][2];
+        float gz = 0.0f;
+        if (WG == 2) {
+            gz = gout[(key << 9) | (uint32_t)tid];
+        } else {
 #pragma unroll
-                for (int t0 = 0; t0 < 27; t0 += 9) {
-                    uint4 val[9];
-#pragma unroll
-                    for (int jj = 0; jj < 9; ++jj) {
-                        const int tap = t0 + jj;
-                        const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                        val[jj] = make_uint4(0u, 0u, 0u, 0u);
-                        const uint32_t u = have ? bw_active(G, ci + dil * dx, cj + dil * dy, ck + dil * dz) : 0xFFFFFFFFu;
-                        if (u != 0xFFFFFFFFu) val[jj] = *reinterpret_cast<const uint4*>(ain + (size_t)u * 16 + h * 8);
-                    }
-#pragma unroll
-                    for (int jj = 0; jj < 9; ++jj) *reinterpret_cast<uint4*>(dst + (t0 + jj) * (kBwRows * 32)) = val[jj];
-                }
+            for (int m = 0; m < 2; ++m) {
+                const int e = tid + m * kBwThreads;
+                const float4* p = reinterpret_cast<const float4*>(gout + (size_t)((key << 9) | (uint32_t)(e >> 1)) * 16 + (e & 1) * 8);
+                g[m][0] = p[0];
+                g[m][1] = p[1];
             }
         }
+        const uint32_t nb1 = around(key1), key2 = key_at(t + 2u * gridDim.x);
+        int ox, oy, oz;
+        tile_origin_tc(key, G.D, ox, oy, oz);
+        const uint32_t st_s = smem_s + (uint32_t)(stage * S::kStage);
+        constexpr int kItems = H * B * B * B;
+#pragma unroll 4
+        for (int w0 = tid - lane; w0 < kItems; w0 += kBwThreads) {  // the same for the whole warp
+            const int e = w0 + lane < kItems ? w0 + lane : kItems - 1;
+            const int h = e % H, v = e / H;
+            const int bx = v % B, by = (v / B) % B, bz = v / (B * B);
+            const int px = bx - DIL, py = by - DIL, pz = bz - DIL;
+            const uint32_t base = __shfl_sync(0xffffffffu, nb, rel_neighbour(px, py, pz));
+            const bool ok = base != kNoTile && ox + px < G.D.nx && oy + py < G.D.ny && oz + pz < G.D.nz;
+            const uint32_t sl = ok ? base | rel_local(px, py, pz) : 0u;
+            if (w0 + lane < kItems)
+                cp_async16(st_s + (uint32_t)((S::row(bz, by) + h) * S::kRow + bx * 16), ain + (size_t)sl * (8 * H) + h * 8, ok);
+        }
+        cp_async_commit();
+        unsigned char* b = st + S::kBox;
+        if (WG == 2) {
+            const float x = gz * scale;
+            const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+            __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(b + tid * 16);
+            row[0] = hi;
+            row[1] = __float2bfloat16_rn(x - __bfloat162float(hi));
+        } else {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int e = tid + m * kBwThreads;
+                const uint4 hi = bf16x8(g[m][0], g[m][1]);
+                unsigned char* row = b + (e & 1) * S::kPart + (e >> 1) * 16;
+                *reinterpret_cast<uint4*>(row) = hi;
+                *reinterpret_cast<uint4*>(row + 2 * S::kPart) = bf16x8_rest(g[m][0], g[m][1], hi);
+            }
+        }
+        key = key1;
+        key1 = key2;
+        nb = nb1;
+    };
+    gather(blockIdx.x, 0);
+    uint32_t i = 0;  // tiles whose MMAs are on their way
+    bool failed = false;
+    // whether the MMAs of this CTA's k-th tile are done
+    auto wait_tile = [&](uint32_t k) {
+        return mbar_wait(mbar_s + 8u * (k % kStages), (k / kStages) & 1u);
+    };
+    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
+        cp_async_wait<0>();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
+        // one decision for the whole CTA
+        if (__syncthreads_or(failed)) break;
         if (tid == 0) {
-            for (int jm = 0; jm < S::kAcc; ++jm) {
-                for (int ks = 0; ks < kBwRows / 16; ++ks) {
-                    // A: row groups 16 jm .. 16 jm + 15 (2 KB apart), voxels 16 ks .. 16 ks + 15
-                    const uint64_t ad = umma_desc(a_s + (uint32_t)(jm * 16 * kBwRows * 16 + ks * 256), 128, kBwRows * 16);
-                    for (int part = 0; part < S::kParts; ++part) {
-                        const uint64_t bd = umma_desc(b_s + (uint32_t)(part * 2 * kBwRows * 16 + ks * 256), 128, kBwRows * 16);
-                        mma_f16(tmem + (uint32_t)(16 * jm), ad, bd, kInstrDescMN, (any || ks > 0 || part > 0) ? 1u : 0u);
+            const uint32_t a_s = smem_s + (i % kStages) * S::kStage, b_s = a_s + S::kBox;
+            for (int ks = 0; ks < 32; ++ks) {
+                // rows y and y + DIL of slice z
+                const int z = ks >> 2, y = ((ks & 3) / DIL) * 2 * DIL + (ks & 3) % DIL;
+                const uint64_t bd = umma_desc(b_s + (uint32_t)((64 * z + 8 * y) * 16), DIL * 128, S::kPart);
+                // a descriptor holds its address in units of 16 B, and the
+                // offsets of the nine (dz, dx) are constants: an addition each
+                const uint64_t ad = umma_desc(a_s + (uint32_t)(S::row(z, y) * S::kRow), H * S::kRow, S::kRow);
+                const uint32_t add = (i > 0 || ks > 0) ? 1u : 0u;
+#pragma unroll
+                for (int j = 0; j < 9; ++j)
+                    mma_f16(tmem + (uint32_t)(S::kN * j), ad + (uint64_t)((S::row(DIL * (j / 3), 0) * S::kRow) / 16 + DIL * (j % 3)), bd,
+                            S::kInstr, add);
+            }
+            mma_commit(mbar_s + 8u * (i % kStages));
+        }
+        ++i;
+        if (t + gridDim.x < n) {
+            // the stage is that of the tile kStages before: its MMAs have to be done
+            if (i >= (uint32_t)kStages && !wait_tile(i - kStages)) failed = true;
+            if (!__any_sync(0xffffffffu, failed)) gather(t + gridDim.x, (int)(i % kStages));
+        }
+    }
+    cp_async_wait<0>();
+    // the last commit covers every MMA before it (bounded: also before TMEM is freed)
+    if (!wait_tile(i - 1)) failed = true;
+    const bool abort = __syncthreads_or(failed) != 0;
+    if (abort && tid == 0) atomicOr(err, 1);
+    if (!abort && warp < 4) {
+        tc_fence_after();
+        for (int j = 0; j < 9; ++j) {
+            float acc[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(S::kN * j), acc);
+            if (S::kN == 32) {
+                float rest[16];
+                tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(S::kN * j + 16), rest);
+#pragma unroll
+                for (int co = 0; co < 16; ++co) acc[co] += rest[co];
+            }
+            const int m = lane + 16 * warp;  // this lane's row of the accumulator, its box row g
+            const int g = m / 8, dy = g / H;
+            if (lane < 16 && dy < 3) {
+                const int tap = 9 * (j / 3) + 3 * dy + j % 3;
+                if (WG == 0) {
+                    // r/s high (0) and low (3) both feed channel 0
+                    const int ch = m & 7;
+                    float* d = dw + (tap * 3 + (ch == 3 ? 0 : ch)) * 16;
+                    if (ch <= 3) {
+#pragma unroll
+                        for (int co = 0; co < 16; ++co)
+                            if (acc[co] != 0.0f) atomicAdd(d + co, acc[co]);
+                    }
+                } else {
+                    const int cin = 8 * (g & 1) + (m & 7);
+                    if (WG == 2) {
+                        const float v = acc[0] + acc[1];
+                        if (v != 0.0f) atomicAdd(dw + tap * 16 + cin, v);
+                    } else {
+                        float* d = dw + (tap * 16 + cin) * 16;
+#pragma unroll
+                        for (int co = 0; co < 16; ++co)
+                            if (acc[co] != 0.0f) atomicAdd(d + co, acc[co]);
                     }
                 }
             }
-            mma_commit(mbar_s);
+            __syncwarp();
         }
-        any = true;
-        pending = true;
-        if (!mbar_wait(mbar_s, phase) && lane == 0) atomicExch(&s_abort, 1);
-        __syncthreads();
-        if (s_abort) break;
-        pending = false;
-        phase ^= 1u;
-        tc_fence_before();
-        __syncthreads();  // the MMAs are done with A and B: the next chunk may overwrite them
-        tc_fence_after();
-    }
-    if (!s_abort && any && warp < 4) {
-        tc_fence_after();
-        for (int jm = 0; jm < S::kAcc; ++jm) {
-            float acc[16];
-            tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(16 * jm), acc);
-            const int m = 32 * warp + lane;
-            const int g = 16 * jm + m / 8;  // this lane's row group
-            if (g >= S::kUsed) continue;
-            if (WG == 0) {
-                // rows r/s high (0) and low (3) both feed channel 0
-                const int c = m & 7;
-                const int cin = c == 3 ? 0 : c;
-                if (c > 3) continue;
-                float* d = dw + (g * 3 + cin) * 16;
-#pragma unroll
-                for (int co = 0; co < 16; ++co)
-                    if (acc[co] != 0.0f) atomicAdd(d + co, acc[co]);
-            } else {
-                const int tap = g >> 1, cin = 8 * (g & 1) + (m & 7);
-                if (WG == 2) {
-                    const float v = acc[0] + acc[1];
-                    if (v != 0.0f) atomicAdd(dw + tap * 16 + cin, v);
-                } else {
-                    float* d = dw + (tap * 16 + cin) * 16;
-#pragma unroll
-                    for (int co = 0; co < 16; ++co)
-                        if (acc[co] != 0.0f) atomicAdd(d + co, acc[co]);
-                }
-            }
-        }
-    }
-    if (s_abort) {
-        if (tid == 0) atomicOr(err, 1);
-        if (pending) mbar_wait(mbar_s, phase);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64) : "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kCols) : "memory");
 }
 
-int lp_mid_dgrad_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, const float* gout, const __nv_bfloat16* ain,
-                    float* gin, int* err, int sms, cudaStream_t st) {
+template <int WG, int DIL>
+static int launch_wgrad_tc(const LpGrid& G, const float* gout, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
+                            const uint32_t* tiles, const uint32_t* d_n, float* dw, int* err, int sms, cudaStream_t st) {
+    using S = WgShape<WG, DIL>;
+    const auto kernel = lp_tc_wgrad_kernel<WG, DIL>;
     static bool attr_set = false;  // per process; the attribute is per function
     if (!attr_set) {
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(lp_tc_dgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgBytes));
+        FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
         attr_set = true;
     }
-    lp_tc_dgrad_kernel<<<sms, kBwThreads, kDgBytes, st>>>(G, wb, dil, gout, ain, gin, err);
+    kernel<<<sms, kBwThreads, S::kBytes, st>>>(G, gout, ain, d_inv_s, sign, tiles, d_n, dw, err);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-
-template <int WG>
-static int launch_wgrad_tc(const LpGrid& G, int dil, const float* gout, const __nv_bfloat16* ain, const float* d_inv_s,
-                           float sign, const uint32_t* tiles, const uint32_t* d_n, float* dw, int* err, int sms,
-                           cudaStream_t st) {
-    static bool attr_set = false;  // per process; the attribute is per function
-    if (!attr_set) {
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(lp_tc_wgrad_kernel<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           WgShape<WG>::kBytes));
-        attr_set = true;
-    }
-    lp_tc_wgrad_kernel<WG><<<sms, kBwThreads, WgShape<WG>::kBytes, st>>>(G, dil, gout, ain, d_inv_s, sign, tiles, d_n, dw,
-                                                                          err);
-    FLIP_CUDA_TRY(cudaGetLastError());
-    return FLIP_OK;
-}
-
-int lp_in_wgrad_tc(const LpGrid& G, int dil, const float* gout, const float* d_inv_s, float* dw, int* err, int sms,
+int lp_in_wgrad_tc(const LpGrid& G, int dil, const float* gout, const float* d_inv_s, void* rows, float* dw, int* err, int sms,
                    cudaStream_t st) {
-    return launch_wgrad_tc<0>(G, dil, gout, nullptr, d_inv_s, 1.0f, G.act_tiles, G.d_nact, dw, err, sms, st);
+    if (dil != 1) return FLIP_ERR_ARG;
+    lp_in_rows_kernel<<<4 * sms, 512, 0, st>>>(G, d_inv_s, static_cast<uint4*>(rows));
+    return launch_wgrad_tc<0, 1>(G, gout, static_cast<const __nv_bfloat16*>(rows), d_inv_s, 1.0f, G.act_tiles, G.d_nact, dw, err,
+                                 sms, st);
 }
 int lp_mid_wgrad_tc(const LpGrid& G, int dil, const float* gout, const __nv_bfloat16* ain, float* dw, int* err, int sms,
                     cudaStream_t st) {
-    return launch_wgrad_tc<1>(G, dil, gout, ain, nullptr, 1.0f, G.act_tiles, G.d_nact, dw, err, sms, st);
+    switch (dil) {
+    case 2: return launch_wgrad_tc<1, 2>(G, gout, ain, nullptr, 1.0f, G.act_tiles, G.d_nact, dw, err, sms, st);
+    case 4: return launch_wgrad_tc<1, 4>(G, gout, ain, nullptr, 1.0f, G.act_tiles, G.d_nact, dw, err, sms, st);
+    default: return FLIP_ERR_ARG;
+    }
 }
 int lp_out_wgrad_tc(const LpGrid& G, int dil, const float* gz, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
                     float* dw, int* err, int sms, cudaStream_t st) {
-    return launch_wgrad_tc<2>(G, dil, gz, ain, d_inv_s, sign, G.out_tiles, G.d_nout, dw, err, sms, st);
+    if (dil != 1) return FLIP_ERR_ARG;
+    return launch_wgrad_tc<2, 1>(G, gz, ain, d_inv_s, sign, G.out_tiles, G.d_nout, dw, err, sms, st);
 }
 
 int lp_small_mid_forward_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, const __nv_bfloat16* in, __nv_bfloat16* out,
@@ -847,9 +843,17 @@ int lp_small_mid_forward_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, c
 int lp_mid_forward_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, const __nv_bfloat16* in, __nv_bfloat16* out,
                       int* err, int sms, cudaStream_t st) {
     switch (dil) {
-    case 1: return launch_mid_tc<1>(G, wb, in, out, err, sms, st);
-    case 2: return launch_mid_tc<2>(G, wb, in, out, err, sms, st);
-    case 4: return launch_mid_tc<4>(G, wb, in, out, err, sms, st);
+    case 1: return launch_mid_tc<1, false>(G, wb, in, nullptr, out, err, sms, st);
+    case 2: return launch_mid_tc<2, false>(G, wb, in, nullptr, out, err, sms, st);
+    case 4: return launch_mid_tc<4, false>(G, wb, in, nullptr, out, err, sms, st);
+    default: return FLIP_ERR_ARG;
+    }
+}
+int lp_mid_dgrad_tc(const LpGrid& G, const __nv_bfloat16* wb, int dil, const float* gout, const __nv_bfloat16* ain,
+                    float* gin, int* err, int sms, cudaStream_t st) {
+    switch (dil) {
+    case 2: return launch_mid_tc<2, true>(G, wb, gout, ain, gin, err, sms, st);
+    case 4: return launch_mid_tc<4, true>(G, wb, gout, ain, gin, err, sms, st);
     default: return FLIP_ERR_ARG;
     }
 }
