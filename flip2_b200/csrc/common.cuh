@@ -53,8 +53,12 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // launch overlaps the predecessor's tail).  Such a kernel calls pdl_wait()
 // before it touches global memory: the call returns once the predecessor
 // has completed and its writes are visible.  In a kernel launched the
-// ordinary way pdl_wait() returns at once.
+// ordinary way pdl_wait() returns at once.  pdl_trigger(), after a kernel's own
+// pdl_wait(), lets the next one start at once: what that does before its
+// pdl_wait() -- weights, indices, allocations, nothing that this kernel writes --
+// then runs beside this kernel.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -404,12 +404,8 @@ __global__ void __launch_bounds__(kSmTcThreads) lp_small_mid_tc_kernel(LpGrid G,
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kSmTcA + kSmTcW);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kSmTcA + kSmTcW + 16);
     __shared__ int s_abort;
-    pdl_wait();
-    if (G.halt && *G.halt) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t nvox = *G.d_nact * 512u;
     const uint32_t v0 = blockIdx.x * kSmTcRows;
-    if (v0 >= nvox) return;
     // weights: global [tap][ci][co] -> per tap [ci/8][co][ci%8]; 27 per thread,
     // loaded in batches of nine before they are stored
 #pragma unroll
@@ -424,46 +420,42 @@ __global__ void __launch_bounds__(kSmTcThreads) lp_small_mid_tc_kernel(LpGrid G,
             *reinterpret_cast<__nv_bfloat16*>(wsm + tap * 512 + (ci >> 3) * 256 + co * 16 + (ci & 7) * 2) = w[j];
         }
     }
-    // A: for each tap, row r = voxel v0 + r, half h = channels 8h .. 8h+7.
-    // A thread keeps one (row, half) and walks the 27 taps: its voxel is
-    // worked out once, and the taps' loads go out nine at a time.
-    {
-        const int h = tid & 1, r = tid >> 1;  // 256 threads = 128 rows x 2 halves
-        const uint32_t vx = v0 + (uint32_t)r;
-        int ci = 0, cj = 0, ck = 0;
-        const bool have = vx < nvox;
-        if (have) {
-            int ox, oy, oz;
-            tile_origin_tc(G.act_tiles[vx >> 9], G.D, ox, oy, oz);
-            const int l = (int)(vx & 511u);
-            ci = ox + (l & 7);
-            cj = oy + ((l >> 3) & 7);
-            ck = oz + (l >> 6);
-        }
-        unsigned char* dst = asm_ + h * (kSmTcRows * 16) + r * 16;
-#pragma unroll
-        for (int t0 = 0; t0 < 27; t0 += 9) {
-            uint4 val[9];
-#pragma unroll
-            for (int j = 0; j < 9; ++j) {
-                const int tap = t0 + j;
-                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                const int gx = ci + dil * dx, gy = cj + dil * dy, gz = ck + dil * dz;
-                val[j] = make_uint4(0u, 0u, 0u, 0u);
-                if (have && gx >= 0 && gy >= 0 && gz >= 0 && gx < G.D.nx && gy < G.D.ny && gz < G.D.nz) {
-                    const uint32_t tt = (uint32_t)((gx >> 3) + G.D.tx * ((gy >> 3) + G.D.ty * (gz >> 3)));
-                    const uint32_t sl = (tt << 9) | (uint32_t)((gx & 7) | ((gy & 7) << 3) | ((gz & 7) << 6));
-                    val[j] = *reinterpret_cast<const uint4*>(in + (size_t)sl * 16 + h * 8);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 9; ++j) *reinterpret_cast<uint4*>(dst + (t0 + j) * (kSmTcRows * 32)) = val[j];
-        }
-    }
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
+    }
+    // A: for each tap, row r = voxel v0 + r, half h = channels 8h .. 8h+7.
+    // A thread keeps one (row, half) and walks the 27 taps: its voxel is
+    // worked out once (the tile list is the problem's, not the previous
+    // kernel's), and all its copies are in flight together.
+    const int h = tid & 1, r = tid >> 1;  // 256 threads = 128 rows x 2 halves
+    const uint32_t nvox = *G.d_nact * 512u;
+    const uint32_t vx = v0 + (uint32_t)r;
+    const bool have = vx < nvox;
+    const uint32_t key = have ? G.act_tiles[vx >> 9] : 0u;
+    int ci, cj, ck;
+    tile_origin_tc(key, G.D, ci, cj, ck);
+    ci += (int)(vx & 7u);
+    cj += (int)((vx >> 3) & 7u);
+    ck += (int)((vx >> 6) & 7u);
+    pdl_wait();
+    pdl_trigger();
+    if (G.halt && *G.halt) return;
+    if (v0 >= nvox) return;
+    {
+        const uint32_t dst = smem_u32(asm_) + (uint32_t)(h * (kSmTcRows * 16) + r * 16);
+#pragma unroll
+        for (int tap = 0; tap < 27; ++tap) {
+            const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+            const int gx = ci + dil * dx, gy = cj + dil * dy, gz = ck + dil * dz;
+            const bool ok = have && gx >= 0 && gy >= 0 && gz >= 0 && gx < G.D.nx && gy < G.D.ny && gz < G.D.nz;
+            const uint32_t tt = (uint32_t)((gx >> 3) + G.D.tx * ((gy >> 3) + G.D.ty * (gz >> 3)));
+            const uint32_t sl = ok ? (tt << 9) | rel_local(gx, gy, gz) : 0u;
+            cp_async16(dst + (uint32_t)(tap * (kSmTcRows * 32)), in + (size_t)sl * 16 + h * 8, ok);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(32)

@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(kMgThreads, kMgCtas) mg_down_kernel(MgLevel F,
     const MgSweep1 P = mg_sweep1(tid);
     const MgOwn O = mg_own(tid);
     pdl_wait();
+    if (SCALE) pdl_trigger();
     if (mg_halted(halt)) return;
     const uint32_t n = *F.d_ntiles;
     uint32_t pc[kQPer];
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(kMgThreads, kMgCtas) mg_sweeps_kernel(MgLevel 
     const MgSweep1 P = mg_sweep1(tid);
     const MgOwn O = mg_own(tid);
     pdl_wait();
+    if (MODE != 0) pdl_trigger();
     if (mg_halted(halt)) return;
     const uint32_t n = *L.d_ntiles;
     const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
