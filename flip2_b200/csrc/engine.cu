@@ -1546,7 +1546,9 @@ static int cap_step(flip_engine* e) {
 static uint32_t cap_step_launches(flip_engine* e) {
     uint32_t k = 2 + (uint32_t)((e->key_bits + 7) / 8) + 1 + 1;  // sort, gather, heads
     k += 1 + (e->has_solid ? 1 : 0) + 3 + 1;                       // P2G .. normalise
-    k += 2 + (e->P.pcg_warm_start ? 1 : 0) + 1 + 1;                // state, init (+ warm), loop condition, record
+    k += 2 + (e->P.pcg_warm_start ? 1 : 0) + 1;                    // state, init (+ warm), record
+    // the resident solve and, where a box may not fit it, its loop's condition
+    k += e->P.pressure_method == 0 ? (resident_always(e) ? 1 : 2) : 1;  // method 2: its loop's condition
     if (e->P.pressure_method == 2) {
         const bool network = e->P.mg_coarse == 0;
         k += 2u * (uint32_t)(e->mg.levels - 1) + 2u * (uint32_t)std::max(0, e->mg.levels - 2) + (network ? 4u : 0u);
@@ -1672,8 +1674,8 @@ static int rec_refresh(flip_engine* e) {
     if (e->P.pressure_method == 2) per_primary = (2u + mg_cycle_launches(e, e->P.mg_coarse == 0, true)) * (uint32_t)chunk + 2u;
     e->launches += (uint32_t)((r.chunks_primary - e->rec_chunks_counted[0]) * per_primary +
                               (r.chunks_plain - e->rec_chunks_counted[1]) * per_plain);
-    // a restart runs the state, init, loop-condition and record kernels of its branch
-    e->launches += (uint32_t)(4u * (r.fallbacks_captured - e->rec_fallbacks_counted));
+    // a restart runs the state, init, resident (and loop-condition) and record kernels of its branch
+    e->launches += (uint32_t)((resident_always(e) ? 4u : 5u) * (r.fallbacks_captured - e->rec_fallbacks_counted));
     e->rec_chunks_counted[0] = r.chunks_primary;
     e->rec_chunks_counted[1] = r.chunks_plain;
     e->rec_fallbacks_counted = r.fallbacks_captured;

@@ -29,7 +29,7 @@ struct PcgState {
     float inv_s;  // 1 / rms(r) over fluid cells: input scale of the learned preconditioner
     int flexible; // 1: FPCG (z = N(r) given), 0: Jacobi PCG
     double zq, nfluid;
-    int chunks;   // chunks the device-side loop has run
+    int chunks;   // chunks the device-side loop has run (not the resident solve)
     double rr_check;  // r.r at the previous true-residual check (bb before the first)
 };
 // flexible CG gives up (done = 4) when the true r.r at a check exceeds this

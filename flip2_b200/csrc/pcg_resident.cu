@@ -662,7 +662,6 @@ __device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* p
         st->iter = iter;
         st->true_checks = true_checks;
         st->next_check = next_check;
-        st->chunks = chunks;
         st->done = lost ? 5 : done;
         st->halt = 1;
         *A.epoch = X.tag + 4u;  // past any tag of a solve that gave up
