@@ -8,7 +8,7 @@
 // Structure (Adinets & Merrill's onesweep):
 //   1. one upfront pass reads every key once and builds all digit histograms
 //      (shared-memory atomics into one histogram per warp);
-//   2. one kernel per 8-bit digit: each CTA claims the next tile of 6144 keys
+//   2. one kernel per 8-bit digit: each CTA claims the next tile of keys
 //      from an atomic counter, ranks its keys per warp with match/ballot,
 //      publishes its per-digit counts and resolves its global offsets with a
 //      decoupled look-back over the predecessor tiles, then scatters through
@@ -20,8 +20,18 @@ namespace flip {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 24;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 6144 keys
+// Keys per thread.  A tile's time is a chain over its thread's keys (load,
+// match, count), so where tiles of kItemsLarge keys leave SMs without one, a sort
+// takes tiles of a quarter.  15-bit keys, large and small tiles: 2,000 keys 21.7
+// and 14.1 us, 30,000 29.8 and 19.4, 262,144 33.9 and 28.6, 500,000 36.8 and 37.0,
+// 2 million 78 and 86 us (more tiles to look back over).
+constexpr int kItemsLarge = 24, kItemsSmall = 6;  // tiles of 6144 and 1536 keys
+constexpr uint64_t kSmallUpTo = 1u << 18;
+static inline int sort_items(uint64_t n) { return n <= kSmallUpTo ? kItemsSmall : kItemsLarge; }
+static inline uint64_t sort_tiles(uint64_t n) {
+    const uint64_t tile = (uint64_t)kSortThreads * sort_items(n);
+    return (n + tile - 1) / tile;
+}
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 4;
 constexpr int kLook = 8;  // predecessors a look-back step reads at once
@@ -37,7 +47,7 @@ struct SortLayout {
 };
 static SortLayout sort_layout(uint64_t n) {
     SortLayout L;
-    uint64_t tiles = (n + kSortTile - 1) / kSortTile;
+    const uint64_t tiles = sort_tiles(n);
     size_t o = 0;
     L.err = o; o = align_up(o + 16, 256);
     L.hist = o; o = align_up(o + sizeof(uint32_t) * kMaxPasses * kRadix, 256);
@@ -127,12 +137,13 @@ __global__ void sort_offsets_kernel(const uint32_t* __restrict__ hist, uint32_t*
 }
 
 // ------------------------------------------------------------ onesweep
-template <bool kIota>
+template <bool kIota, int kItems>
 __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, uint64_t n, int shift, const uint32_t* __restrict__ offsets,
     uint32_t* __restrict__ status, uint32_t* __restrict__ tile_ctr, uint32_t* __restrict__ err, uint32_t spin_limit,
     uint32_t tile_base, uint32_t* __restrict__ head_dense, uint32_t head_limit) {
+    constexpr int kTile = kSortThreads * kItems;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_whist[kSortWarps][kRadix];  // warp counts, then warp offsets within the digit
     __shared__ uint32_t s_blk[kRadix];                // tile-local exclusive offset of each digit
@@ -140,19 +151,19 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(
     __shared__ uint32_t s_scan[kSortWarps + 1];
     extern __shared__ uint32_t s_stage[];  // the tile reordered: keys, then values
     uint32_t* s_keys = s_stage;
-    uint32_t* s_vals = s_stage + kSortTile;
+    uint32_t* s_vals = s_stage + kTile;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u) + tile_base;
     for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) (&s_whist[0][0])[i] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
-    const uint64_t base = (uint64_t)tile * kSortTile;
+    const uint64_t base = (uint64_t)tile * kTile;
 
-    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+    uint32_t key[kItems], val[kItems], rank[kItems];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        uint64_t idx = base + (uint64_t)warp * (kSortItems * 32) + i * 32 + lane;
+    for (int i = 0; i < kItems; ++i) {
+        uint64_t idx = base + (uint64_t)warp * (kItems * 32) + i * 32 + lane;
         if (idx < n) {
             key[i] = kin[idx];
             val[i] = kIota ? (uint32_t)idx : vin[idx];
@@ -164,7 +175,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(
     // stable per-warp ranking, item order = input order
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < kItems; ++i) {
         uint32_t d = (key[i] >> shift) & 0xFFu;
         uint32_t peers = __match_any_sync(0xffffffffu, d);
         uint32_t before = __popc(peers & lt);
@@ -231,14 +242,14 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(
     __syncthreads();
 
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < kItems; ++i) {
         uint32_t dd = (key[i] >> shift) & 0xFFu;
         uint32_t pos = s_blk[dd] + s_whist[warp][dd] + rank[i];
         s_keys[pos] = key[i];
         s_vals[pos] = val[i];
     }
     __syncthreads();
-    const uint32_t valid = (uint32_t)((n - base) < (uint64_t)kSortTile ? (n - base) : kSortTile);
+    const uint32_t valid = (uint32_t)((n - base) < (uint64_t)kTile ? (n - base) : kTile);
     for (uint32_t j = tid; j < valid; j += kSortThreads) {
         uint32_t k = s_keys[j];
         uint32_t dd = (k >> shift) & 0xFFu;
@@ -252,6 +263,22 @@ __global__ void __launch_bounds__(kSortThreads, 3) onesweep_kernel(
             if (head_dense && (j == 0 || s_keys[j - 1] != k) && k < head_limit) atomicMin(head_dense + k, o);
         }
     }
+}
+
+template <bool kIota, int kItems>
+static int launch_onesweep(unsigned grid, int dev, const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
+                           uint64_t n, int shift, const uint32_t* offsets, uint32_t* status, uint32_t* ctr, uint32_t* err,
+                           uint32_t spin_limit, uint32_t tile_base, uint32_t* head_dense, uint32_t head_limit, cudaStream_t s) {
+    constexpr int kStage = 2 * kSortThreads * kItems * (int)sizeof(uint32_t);
+    // the staging buffer may exceed the default 48 KB (once per device)
+    static bool stage_attr[64] = {};
+    if (dev >= 0 && dev < 64 && !stage_attr[dev]) {
+        FLIP_CUDA_TRY(cudaFuncSetAttribute(onesweep_kernel<kIota, kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStage));
+        stage_attr[dev] = true;
+    }
+    onesweep_kernel<kIota, kItems><<<grid, kSortThreads, kStage, s>>>(kin, vin, kout, vout, n, shift, offsets, status, ctr, err,
+                                                                      spin_limit, tile_base, head_dense, head_limit);
+    return FLIP_OK;
 }
 
 }  // namespace flip
@@ -285,7 +312,7 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
     uint32_t* av = (uint32_t*)(S + L.alt_v);
     const int passes = (key_bits + 7) / 8;
 
-    const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
+    const uint64_t tiles = sort_tiles(n);
     if (tile_base >= tiles) {
         set_error_text("flip_sort_pairs: tile_base beyond the tile count");
         return FLIP_ERR_ARG;
@@ -296,15 +323,6 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
     FLIP_CUDA_TRY(cudaMemsetAsync(S, 0, L.status + sizeof(uint32_t) * passes * tiles * kRadix, s));
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
-    // the staging buffer may exceed the default 48 KB (once per device)
-    static bool stage_attr[64] = {};
-    if (dev >= 0 && dev < 64 && !stage_attr[dev]) {
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(onesweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           2 * kSortTile * (int)sizeof(uint32_t)));
-        FLIP_CUDA_TRY(cudaFuncSetAttribute(onesweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           2 * kSortTile * (int)sizeof(uint32_t)));
-        stage_attr[dev] = true;
-    }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // one wave: as many blocks as are resident at once
     const size_t hsmem = sizeof(uint32_t) * kSortWarps * passes * kRadix;
@@ -328,13 +346,13 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
         uint32_t* ov = to_out ? vals_out : av;
         uint32_t* pstat = status + (size_t)p * tiles * kRadix;
         uint32_t* hd = p == passes - 1 ? head_dense : nullptr;
-        constexpr int kStage = 2 * kSortTile * (int)sizeof(uint32_t);
-        if (p == 0 && cv == nullptr)
-            onesweep_kernel<true><<<grid, kSortThreads, kStage, s>>>(ck, nullptr, ok, ov, n, 8 * p, offs + p * kRadix, pstat,
-                                                                ctr + p, err, spin_limit, tile_base, hd, head_limit);
-        else
-            onesweep_kernel<false><<<grid, kSortThreads, kStage, s>>>(ck, cv, ok, ov, n, 8 * p, offs + p * kRadix, pstat,
-                                                                 ctr + p, err, spin_limit, tile_base, hd, head_limit);
+        const bool iota = p == 0 && cv == nullptr;
+        const bool small = sort_items(n) == kItemsSmall;
+        const auto launch = iota ? (small ? launch_onesweep<true, kItemsSmall> : launch_onesweep<true, kItemsLarge>)
+                                 : (small ? launch_onesweep<false, kItemsSmall> : launch_onesweep<false, kItemsLarge>);
+        const int rc = launch(grid, dev, ck, cv, ok, ov, n, 8 * p, offs + p * kRadix, pstat, ctr + p, err, spin_limit, tile_base, hd,
+                              head_limit, s);
+        if (rc != FLIP_OK) return rc;
         ck = ok;
         cv = ov;
     }
