@@ -27,9 +27,8 @@ constexpr int kSortWarps = kSortThreads / 32;
 // 2 million 78 and 86 us (more tiles to look back over).
 constexpr int kItemsLarge = 24, kItemsSmall = 6;  // tiles of 6144 and 1536 keys
 constexpr uint64_t kSmallUpTo = 1u << 18;
-static inline int sort_items(uint64_t n) { return n <= kSmallUpTo ? kItemsSmall : kItemsLarge; }
-static inline uint64_t sort_tiles(uint64_t n) {
-    const uint64_t tile = (uint64_t)kSortThreads * sort_items(n);
+static inline uint64_t sort_tiles(uint64_t n, int items) {
+    const uint64_t tile = (uint64_t)kSortThreads * items;
     return (n + tile - 1) / tile;
 }
 constexpr int kRadix = 256;
@@ -45,9 +44,8 @@ static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 struct SortLayout {
     size_t err, hist, offsets, ctr, status, alt_k, alt_v, total;
 };
-static SortLayout sort_layout(uint64_t n) {
+static SortLayout sort_layout(uint64_t n, uint64_t tiles) {
     SortLayout L;
-    const uint64_t tiles = sort_tiles(n);
     size_t o = 0;
     L.err = o; o = align_up(o + 16, 256);
     L.hist = o; o = align_up(o + sizeof(uint32_t) * kMaxPasses * kRadix, 256);
@@ -285,7 +283,12 @@ static int launch_onesweep(unsigned grid, int dev, const uint32_t* kin, const ui
 
 using namespace flip;
 
-extern "C" size_t flip_sort_pairs_scratch_bytes(uint64_t n) { return sort_layout(n).total; }
+// room for the small tiles of any count up to n, so that a scratch sized for a
+// count holds every smaller sort
+extern "C" size_t flip_sort_pairs_scratch_bytes(uint64_t n) {
+    const uint64_t small = sort_tiles(n < kSmallUpTo ? n : kSmallUpTo, kItemsSmall), large = sort_tiles(n, kItemsLarge);
+    return sort_layout(n, small > large ? small : large).total;
+}
 
 int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out, uint32_t* vals_out,
                         uint64_t n, int key_bits, void* scratch, size_t scratch_bytes, cudaStream_t s,
@@ -297,7 +300,13 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
         set_error_text("flip_sort_pairs: bad argument (null pointer, key_bits outside 1..32 or n >= 2^30)");
         return FLIP_ERR_ARG;
     }
-    SortLayout L = sort_layout(n);
+    // small tiles where their look-back words fit
+    int items = kItemsSmall;
+    SortLayout L = sort_layout(n, sort_tiles(n, items));
+    if (n > kSmallUpTo || scratch_bytes < L.total) {
+        items = kItemsLarge;
+        L = sort_layout(n, sort_tiles(n, items));
+    }
     if (scratch_bytes < L.total) {
         set_error_text("flip_sort_pairs: scratch too small");
         return FLIP_ERR_ARG;
@@ -312,7 +321,7 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
     uint32_t* av = (uint32_t*)(S + L.alt_v);
     const int passes = (key_bits + 7) / 8;
 
-    const uint64_t tiles = sort_tiles(n);
+    const uint64_t tiles = sort_tiles(n, items);
     if (tile_base >= tiles) {
         set_error_text("flip_sort_pairs: tile_base beyond the tile count");
         return FLIP_ERR_ARG;
@@ -347,7 +356,7 @@ int flip::sort_pairs_ex(const uint32_t* keys_in, const uint32_t* vals_in, uint32
         uint32_t* pstat = status + (size_t)p * tiles * kRadix;
         uint32_t* hd = p == passes - 1 ? head_dense : nullptr;
         const bool iota = p == 0 && cv == nullptr;
-        const bool small = sort_items(n) == kItemsSmall;
+        const bool small = items == kItemsSmall;
         const auto launch = iota ? (small ? launch_onesweep<true, kItemsSmall> : launch_onesweep<true, kItemsLarge>)
                                  : (small ? launch_onesweep<false, kItemsSmall> : launch_onesweep<false, kItemsLarge>);
         const int rc = launch(grid, dev, ck, cv, ok, ov, n, 8 * p, offs + p * kRadix, pstat, ctr + p, err, spin_limit, tile_base, hd,

@@ -27,12 +27,15 @@ def test_sort_sizes(n, bits, distinct):
     def p(t):
         return C.c_void_p(t.data_ptr() if t is not None else None)
 
-    for payload in (None, vals):
+    # a scratch sized for more keys holds fewer, and the look-back words of
+    # large tiles (1 KB a digit pass and 6144 keys) are enough for any count
+    assert L.flip_sort_pairs_scratch_bytes(C.c_uint64(n + 5000)) >= nbytes
+    large = nbytes - 4 * 1024 * max(0, -(-min(n, 1 << 18) // 1536) - -(-n // 6144))
+    for payload, room in ((None, nbytes), (vals, nbytes), (vals, large)):
         ko, vo = torch.empty_like(keys), torch.empty_like(keys)
-        rc = L.flip_sort_pairs(p(keys), p(payload), p(ko), p(vo), C.c_uint64(n), bits, p(scratch), C.c_size_t(nbytes), None)
+        rc = L.flip_sort_pairs(p(keys), p(payload), p(ko), p(vo), C.c_uint64(n), bits, p(scratch), C.c_size_t(room), None)
         torch.cuda.synchronize()
         assert rc == 0
         assert torch.equal(ko.long(), want)
         assert torch.equal(vo.long(), perm if payload is None else vals.long()[perm])
-        # one byte less scratch than asked for stays an error
-        assert L.flip_sort_pairs(p(keys), p(payload), p(ko), p(vo), C.c_uint64(n), bits, p(scratch), C.c_size_t(nbytes - 1), None) != 0
+    assert L.flip_sort_pairs(p(keys), None, p(ko), p(vo), C.c_uint64(n), bits, p(scratch), C.c_size_t(large - 1), None) != 0
