@@ -52,6 +52,15 @@ __device__ __forceinline__ void load16(const __nv_bfloat16* a, uint32_t u, float
         x[8 + 2 * m] = f1.x; x[8 + 2 * m + 1] = f1.y;
     }
 }
+__device__ __forceinline__ void unpack8(const uint4& q, float* x) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const float2 f = __bfloat1622float2(h[m]);
+        x[2 * m] = f.x;
+        x[2 * m + 1] = f.y;
+    }
+}
 __device__ __forceinline__ void store16(__nv_bfloat16* a, uint32_t u, const float (&x)[16]) {
     uint4 q0, q1;
     __nv_bfloat162* h0 = reinterpret_cast<__nv_bfloat162*>(&q0);
@@ -67,39 +76,77 @@ __device__ __forceinline__ void store16(__nv_bfloat16* a, uint32_t u, const floa
 }
 
 // ---------------------------------------------------------------- forward
+// The first and the last layer (dilation 1) on CUDA cores, FP32 sums: a CTA of
+// 256 threads stages a tile's 10^3 input box in shared memory (zero where there
+// are no activations) and a thread computes two voxels, four z-slices apart,
+// so that a weight read serves both.  Bound by FMAs and shared memory reads.  A
+// thread a voxel with a tile lookup and global reads per tap took 213, 166 and
+// 203 us at 128^3 (first layer, last layer, the last one's input gradient), this
+// 138, 101 and 76 us.
+constexpr int kEdgeThreads = 256;
+constexpr int kEdgeBox = 10;
+constexpr int kEdgeVox = kEdgeBox * kEdgeBox * kEdgeBox;
+constexpr int kEdgeCtas = 4;  // of the launches' two CTAs per SM: one stages while others compute
+__device__ __forceinline__ int edge_at(int x, int y, int z) { return (x + 1) + kEdgeBox * ((y + 1) + kEdgeBox * (z + 1)); }
+// F(box voxel, its slot or UINT32_MAX) for every voxel of a tile's box
+template <class Fn>
+__device__ __forceinline__ void edge_stage(const LpGrid& G, uint32_t key, Fn F) {
+    int ox, oy, oz;
+    tile_origin(key, G.D, ox, oy, oz);
+    for (int e = threadIdx.x; e < kEdgeVox; e += kEdgeThreads)
+        F(e, active_slot(ox - 1 + e % kEdgeBox, oy - 1 + (e / kEdgeBox) % kEdgeBox, oz - 1 + e / (kEdgeBox * kEdgeBox), G));
+}
+// acc[v][c] += x[v] w[c], 16 channels of two voxels
+__device__ __forceinline__ void edge_fma(float (&acc)[2][16], const float* w, const float (&x)[2]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 w4 = *reinterpret_cast<const float4*>(w + 4 * q);
+        const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) acc[v][4 * q + c] = fmaf(wv[c], x[v], acc[v][4 * q + c]);
+    }
+}
+
 // layer 0: 3 -> 16, ReLU
-__global__ void __launch_bounds__(512) lp_in_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, int dil,
-                                                    const float* __restrict__ d_inv_s, __nv_bfloat16* __restrict__ out) {
+__global__ void __launch_bounds__(kEdgeThreads) lp_in_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb,
+                                                             const float* __restrict__ d_inv_s, __nv_bfloat16* __restrict__ out) {
     if (G.halt && *G.halt) return;
-    __shared__ float W[27 * 3 * 16];
-    for (int i = threadIdx.x; i < 27 * 3 * 16; i += 512) W[i] = __bfloat162float(wb[i]);
-    __syncthreads();
+    __shared__ __align__(16) float W[27 * 3 * 16];
+    __shared__ float X[3][kEdgeVox];
+    for (int i = threadIdx.x; i < 27 * 3 * 16; i += kEdgeThreads) W[i] = __bfloat162float(wb[i]);
     const float inv_s = *d_inv_s;
     const uint32_t n = *G.d_nact;
     const int li = threadIdx.x & 7, lj = (threadIdx.x >> 3) & 7, lk = threadIdx.x >> 6;
     for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
         const uint32_t key = G.act_tiles[t];
-        int ox, oy, oz;
-        tile_origin(key, G.D, ox, oy, oz);
-        const int i = ox + li, j = oy + lj, k = oz + lk;
-        float acc[16];
+        __syncthreads();
+        edge_stage(G, key, [&](int e, uint32_t u) {
+            float in[3] = {0.0f, 0.0f, 0.0f};
+            if (u != 0xFFFFFFFFu) input_channels(G, u, inv_s, in);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+            for (int ci = 0; ci < 3; ++ci) X[ci][e] = in[ci];
+        });
+        __syncthreads();
+        float acc[2][16] = {};
+#pragma unroll 1
         for (int tap = 0; tap < 27; ++tap) {
             int dx, dy, dz;
             tap_off(tap, dx, dy, dz);
-            const uint32_t u = active_slot(i + dil * dx, j + dil * dy, k + dil * dz, G);
-            if (u == 0xFFFFFFFFu) continue;
-            float in[3];
-            input_channels(G, u, inv_s, in);
+            const int at = edge_at(li + dx, lj + dy, lk + dz);
 #pragma unroll
-            for (int ci = 0; ci < 3; ++ci)
-#pragma unroll
-                for (int co = 0; co < 16; ++co) acc[co] = fmaf(W[(tap * 3 + ci) * 16 + co], in[ci], acc[co]);
+            for (int ci = 0; ci < 3; ++ci) {
+                const float x[2] = {X[ci][at], X[ci][at + 4 * kEdgeBox * kEdgeBox]};
+                edge_fma(acc, W + (tap * 3 + ci) * 16, x);
+            }
         }
 #pragma unroll
-        for (int c = 0; c < 16; ++c) acc[c] = fmaxf(acc[c], 0.0f);
-        store16(out, (key << 9) | threadIdx.x, acc);
+        for (int v = 0; v < 2; ++v) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc[v][c] = fmaxf(acc[v][c], 0.0f);
+            store16(out, (key << 9) | (threadIdx.x + 256u * v), acc[v]);
+        }
     }
 }
 
@@ -141,37 +188,56 @@ __global__ void __launch_bounds__(512) lp_mid_kernel(LpGrid G, const __nv_bfloat
 
 // layer 3: 16 -> 1 on fluid cells.  raw: z = f (the zero-residual pass);
 // else z = s (f - f0[v]) with f0 optional
-__global__ void __launch_bounds__(512) lp_out_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, int dil,
-                                                     const __nv_bfloat16* __restrict__ in, const float* __restrict__ d_inv_s,
-                                                     const float* __restrict__ f0, int raw, float* __restrict__ z) {
+__global__ void __launch_bounds__(kEdgeThreads) lp_out_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb,
+                                                              const __nv_bfloat16* __restrict__ in,
+                                                              const float* __restrict__ d_inv_s, const float* __restrict__ f0,
+                                                              int raw, float* __restrict__ z) {
     if (G.halt && *G.halt) return;
-    __shared__ float W[27 * 16];
-    for (int i = threadIdx.x; i < 27 * 16; i += 512) W[i] = __bfloat162float(wb[i]);
-    __syncthreads();
+    __shared__ __align__(16) float W[27 * 16];
+    __shared__ uint4 X[2][kEdgeVox];  // channels 0-7, 8-15
+    for (int i = threadIdx.x; i < 27 * 16; i += kEdgeThreads) W[i] = __bfloat162float(wb[i]);
     const float s = 1.0f / *d_inv_s;
     const uint32_t n = *G.d_nout;
     const int li = threadIdx.x & 7, lj = (threadIdx.x >> 3) & 7, lk = threadIdx.x >> 6;
     for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
         const uint32_t key = G.out_tiles[t];
-        const uint32_t v = (key << 9) | threadIdx.x;
-        float acc = 0.0f;
-        if (G.type[v] == kFluid) {
-            int ox, oy, oz;
-            tile_origin(key, G.D, ox, oy, oz);
-            const int i = ox + li, j = oy + lj, k = oz + lk;
-            for (int tap = 0; tap < 27; ++tap) {
-                int dx, dy, dz;
-                tap_off(tap, dx, dy, dz);
-                const uint32_t u = active_slot(i + dil * dx, j + dil * dy, k + dil * dz, G);
-                if (u == 0xFFFFFFFFu) continue;
-                float x[16];
-                load16(in, u, x);
-#pragma unroll
-                for (int ci = 0; ci < 16; ++ci) acc = fmaf(W[tap * 16 + ci], x[ci], acc);
+        __syncthreads();
+        edge_stage(G, key, [&](int e, uint32_t u) {
+            uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+            if (u != 0xFFFFFFFFu) {
+                const uint4* p = reinterpret_cast<const uint4*>(in + (size_t)u * 16);
+                a = p[0];
+                b = p[1];
             }
-            if (!raw) acc = (acc - (f0 ? f0[v] : 0.0f)) * s;
+            X[0][e] = a;
+            X[1][e] = b;
+        });
+        __syncthreads();
+        float acc[2] = {0.0f, 0.0f};
+#pragma unroll 1
+        for (int tap = 0; tap < 27; ++tap) {
+            int dx, dy, dz;
+            tap_off(tap, dx, dy, dz);
+            const int at = edge_at(li + dx, lj + dy, lk + dz);
+            __align__(16) float w[16];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) *reinterpret_cast<float4*>(w + 4 * q) = *reinterpret_cast<const float4*>(W + tap * 16 + 4 * q);
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                float x[16];
+                unpack8(X[0][at + 4 * kEdgeBox * kEdgeBox * v], x);
+                unpack8(X[1][at + 4 * kEdgeBox * kEdgeBox * v], x + 8);
+#pragma unroll
+                for (int ci = 0; ci < 16; ++ci) acc[v] = fmaf(w[ci], x[ci], acc[v]);
+            }
         }
-        z[v] = acc;
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const uint32_t u = (key << 9) | (threadIdx.x + 256u * v);
+            float o = 0.0f;
+            if (G.type[u] == kFluid) o = raw ? acc[v] : (acc[v] - (f0 ? f0[u] : 0.0f)) * s;
+            z[u] = o;
+        }
     }
 }
 
@@ -243,15 +309,6 @@ __device__ __forceinline__ void small_gather16(const LpGrid& G, const SmallVoxel
     for (int m = 0; m < kPer; ++m) {
         const int e = threadIdx.x + m * kSmallThreads;
         if (e < kItems) X[e] = val[m];
-    }
-}
-__device__ __forceinline__ void unpack8(const uint4& q, float* x) {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-        const float2 f = __bfloat1622float2(h[m]);
-        x[2 * m] = f.x;
-        x[2 * m + 1] = f.y;
     }
 }
 
@@ -398,40 +455,45 @@ int lp_small_forward(const LpNet& net, const LpGrid& G, uint32_t ntiles, const f
 // --------------------------------------------------------------- backward
 // dL/d(layer-2 activations) from dL/dz: G2[u][ci] = relu'(A2[u][ci]) *
 // sum_tap W3[tap][ci] * s * gz(u - dil*off); gz is zero off fluid cells
-__global__ void __launch_bounds__(512) lp_out_dgrad_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, int dil,
-                                                           const float* __restrict__ gz, const __nv_bfloat16* __restrict__ a2,
-                                                           const float* __restrict__ d_inv_s, float sign,
-                                                           float* __restrict__ g2) {
-    __shared__ float W[27 * 16];
-    for (int i = threadIdx.x; i < 27 * 16; i += 512) W[i] = __bfloat162float(wb[i]);
-    __syncthreads();
+__global__ void __launch_bounds__(kEdgeThreads) lp_out_dgrad_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb,
+                                                                    const float* __restrict__ gz,
+                                                                    const __nv_bfloat16* __restrict__ a2,
+                                                                    const float* __restrict__ d_inv_s, float sign,
+                                                                    float* __restrict__ g2) {
+    __shared__ __align__(16) float W[27 * 16];
+    __shared__ float X[kEdgeVox];
+    for (int i = threadIdx.x; i < 27 * 16; i += kEdgeThreads) W[i] = __bfloat162float(wb[i]);
     const float s = sign / *d_inv_s;
     const uint32_t n = *G.d_nact;
     const int li = threadIdx.x & 7, lj = (threadIdx.x >> 3) & 7, lk = threadIdx.x >> 6;
     for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
         const uint32_t key = G.act_tiles[t];
-        int ox, oy, oz;
-        tile_origin(key, G.D, ox, oy, oz);
-        const int i = ox + li, j = oy + lj, k = oz + lk;
-        const uint32_t u = (key << 9) | threadIdx.x;
-        float acc[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+        __syncthreads();
+        edge_stage(G, key, [&](int e, uint32_t u) { X[e] = u != 0xFFFFFFFFu ? gz[u] : 0.0f; });
+        __syncthreads();
+        float acc[2][16] = {};
+#pragma unroll 3
         for (int tap = 0; tap < 27; ++tap) {
             int dx, dy, dz;
             tap_off(tap, dx, dy, dz);
-            const uint32_t v = active_slot(i - dil * dx, j - dil * dy, k - dil * dz, G);
-            if (v == 0xFFFFFFFFu) continue;
-            const float g = gz[v];
-            if (g == 0.0f) continue;
-#pragma unroll
-            for (int ci = 0; ci < 16; ++ci) acc[ci] = fmaf(W[tap * 16 + ci], g, acc[ci]);
+            const int at = edge_at(li - dx, lj - dy, lk - dz);
+            const float x[2] = {X[at], X[at + 4 * kEdgeBox * kEdgeBox]};
+            edge_fma(acc, W + tap * 16, x);
         }
-        float a[16];
-        load16(a2, u, a);
-        float* out = g2 + (size_t)u * 16;
 #pragma unroll
-        for (int ci = 0; ci < 16; ++ci) out[ci] = (a[ci] > 0.0f) ? acc[ci] * s : 0.0f;
+        for (int v = 0; v < 2; ++v) {
+            const uint32_t u = (key << 9) | (threadIdx.x + 256u * v);
+            float a[16];
+            load16(a2, u, a);
+            float4* o = reinterpret_cast<float4*>(g2 + (size_t)u * 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float r[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) r[c] = (a[4 * q + c] > 0.0f) ? acc[v][4 * q + c] * s : 0.0f;
+                o[q] = make_float4(r[0], r[1], r[2], r[3]);
+            }
+        }
     }
 }
 
@@ -558,7 +620,8 @@ __global__ void lp_to_bf16_kernel(const float* __restrict__ w, __nv_bfloat16* __
 // the three hidden layers into acts[0..2]
 static int lp_hidden(const LpNet& net, const LpGrid& G, const float* d_inv_s, __nv_bfloat16* const* acts, int grid,
                      cudaStream_t st) {
-    lp_in_kernel<<<grid, 512, 0, st>>>(G, net.wb + kLpWOff[0], net.dil[0], d_inv_s, acts[0]);
+    if (net.dil[0] != 1) return FLIP_ERR_ARG;
+    lp_in_kernel<<<kEdgeCtas * grid, kEdgeThreads, 0, st>>>(G, net.wb + kLpWOff[0], d_inv_s, acts[0]);
     if (net.tensor_cores) {
         int rc = lp_mid_forward_tc(G, net.wb + kLpWOff[1], net.dil[1], acts[0], acts[1], net.err, net.sms, st);
         if (rc == FLIP_OK) rc = lp_mid_forward_tc(G, net.wb + kLpWOff[2], net.dil[2], acts[1], acts[2], net.err, net.sms, st);
@@ -576,7 +639,8 @@ int lp_bias_dev(const LpNet& net, const LpGrid& G, const float* d_inv_s, float* 
     G0.r = nullptr;
     int rc = lp_hidden(net, G0, d_inv_s, net.actz, grid, st);
     if (rc != FLIP_OK) return rc;
-    lp_out_kernel<<<grid, 512, 0, st>>>(G0, net.wb + kLpWOff[3], net.dil[3], net.actz[2], d_inv_s, nullptr, 1, f0);
+    if (net.dil[3] != 1) return FLIP_ERR_ARG;
+    lp_out_kernel<<<kEdgeCtas * grid, kEdgeThreads, 0, st>>>(G0, net.wb + kLpWOff[3], net.actz[2], d_inv_s, nullptr, 1, f0);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
@@ -585,7 +649,8 @@ int lp_forward_dev(const LpNet& net, const LpGrid& G, const float* d_inv_s, cons
                    cudaStream_t st) {
     int rc = lp_hidden(net, G, d_inv_s, net.act, grid, st);
     if (rc != FLIP_OK) return rc;
-    lp_out_kernel<<<grid, 512, 0, st>>>(G, net.wb + kLpWOff[3], net.dil[3], net.act[2], d_inv_s, f0, 0, z);
+    if (net.dil[3] != 1) return FLIP_ERR_ARG;
+    lp_out_kernel<<<kEdgeCtas * grid, kEdgeThreads, 0, st>>>(G, net.wb + kLpWOff[3], net.act[2], d_inv_s, f0, 0, z);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
@@ -601,7 +666,8 @@ static int lp_backward_path(LpNet& net, const LpGrid& G, const float* d_inv_s, c
         lp_wgrad_kernel<2, 16, 1><<<grid, 512, 0, st>>>(G, net.dil[3], gz, acts[2], d_inv_s, sign, G.out_tiles, G.d_nout,
                                                         net.g + kLpWOff[3]);
     }
-    lp_out_dgrad_kernel<<<grid, 512, 0, st>>>(G, net.wb + kLpWOff[3], net.dil[3], gz, acts[2], d_inv_s, sign, net.gact);
+    if (net.dil[3] != 1) return FLIP_ERR_ARG;
+    lp_out_dgrad_kernel<<<kEdgeCtas * grid, kEdgeThreads, 0, st>>>(G, net.wb + kLpWOff[3], gz, acts[2], d_inv_s, sign, net.gact);
     if (net.tensor_cores) {
         // layer 2 (16 -> 16): Gout = gact (wrt act[2]), input act[1]; then layer 1
         int rc = lp_mid_wgrad_tc(G, net.dil[2], net.gact, acts[1], net.g + kLpWOff[2], net.err, net.sms, st);
