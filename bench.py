@@ -36,6 +36,7 @@ WORKLOAD = ("dam-break 256^3 voxels (cell 1/256), block 0.5x0.5x1, 8 jittered pa
 # algorithmic bytes of one PCG iteration per active voxel, fused minimum:
 # matvec+pAp 9 B, x/r/z update with r.z 28 B, direction update 12 B
 PCG_BYTES_PER_VOXEL = 49.0
+RESIDENT_TILES = 88  # tiles per SM that the resident Jacobi-PCG solve holds
 # one learned multilevel FCG iteration on the fine level: direction+matvec and
 # update 49 B, V-cycle down (code, r in; t, coarse r out) 9.5 B and up (code,
 # r, t in; z out) 12.5 B, plus q in 4 B for the FCG dot products the up
@@ -570,11 +571,13 @@ def main():
             traffic = traffic * voxels
     except (OSError, ValueError):
         pass
-    if c5:
-        traffic = None  # the ncu traffic figure covers the Jacobi-PCG iteration only
+    resident = fluid_tiles <= RESIDENT_TILES * torch.cuda.get_device_properties(dev).multi_processor_count
+    if c5 or resident:
+        traffic = None  # the ncu traffic figure covers the two-kernel Jacobi-PCG iteration only
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic,
                 "kernel": ("learned multilevel FCG iteration (direction+matvec, update, V-cycle with the FCG dot fused)" if c5 else
+                           "pcg iteration (resident kernel: vectors on the chip, so the fraction of the streamed minimum passes 1)" if resident else
                            "pcg iteration (matvec+pAp, x/r update with r.r and r.z, direction)"),
                 "algorithmic_bytes": "%d B per active voxel per iteration x %d voxels" % (per_voxel, voxels),
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6650 GB/s"}
