@@ -410,6 +410,8 @@ extern "C" int flip_set_domain(flip_engine* e, double nx, double ny, double nz, 
         add((void**)&e->d_frame, sizeof(FrameState));
         add((void**)&e->pcg.partials, sizeof(double) * 4 * kPcgBlocks);
         e->pcg.ctas = (uint32_t)std::min<uint64_t>(std::min(e->sms, kResidentMaxCtas), (e->ntiles_total + 3) / 4);
+        e->pcg.cluster = false;
+        if (e->ntiles_total <= 4ull * e->pcg.ctas) E_TRY(nat_pcg_cluster(e->pcg.ctas, &e->pcg.cluster));
         e->pcg.mail_tiles = (uint32_t)std::min<uint64_t>(e->ntiles_total, kResidentTiles * e->pcg.ctas);
         add((void**)&e->pcg.slots, 8 * kPcgSlotWords * 4 * (size_t)e->pcg.ctas);
         add((void**)&e->pcg.epoch, sizeof(uint32_t));

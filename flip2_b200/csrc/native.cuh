@@ -64,6 +64,7 @@ struct PcgBuffers {
     PcgState* st;
     double* partials;  // [4][kPcgBlocks]
     uint32_t ctas;     // CTAs of the resident solve: one per SM, and one per four tiles at most
+    bool cluster;      // ... and they run as one cluster (nat_pcg_cluster)
     unsigned long long* slots;  // its packets, [2][2][ctas][kPcgSlotWords]
     uint32_t* epoch;   // the last tag the resident solve used
     float* far;        // its faces without room on the chip: 768 floats a tile
@@ -204,8 +205,10 @@ int nat_launch_pcgw_iteration(const uint32_t* tiles, const uint32_t* d_ntiles, c
                               cudaStream_t s);
 int nat_launch_pcgw_check(const uint32_t* tiles, const uint32_t* d_ntiles, const NatDims& D, PcgBuffers& B,
                           cudaStream_t s);
-// the whole plain solve after nat_launch_pcgw_init in one cooperative kernel,
-// for at most kResidentTiles tiles per CTA: the
+// whether a solve of `ctas` CTAs, four tiles each at most, runs as one cluster
+int nat_pcg_cluster(uint32_t ctas, bool* fits);
+// the whole plain solve after nat_launch_pcgw_init in one cooperative kernel
+// (or one cluster), for at most kResidentTiles tiles per CTA: the
 // iterations in chunks of `chunk`, the true-residual checks between chunks,
 // at most `limit` chunks.  With more tiles it returns at once and leaves
 // st->done 0; a reduction that gives up sets DEVERR_GRID_TIMEOUT in *err
