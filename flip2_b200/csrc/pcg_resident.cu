@@ -1,5 +1,5 @@
 // pcg_resident.cu -- the whole Jacobi-PCG solve as one cooperative kernel
-// that keeps the solver's vectors on the chip.
+// (small boxes: one cluster) that keeps the solver's vectors on the chip.
 //
 // A CTA per SM owns a run of consecutive tiles for the whole solve.  p of its
 // tiles always lives in shared memory; w = D^-1 r, t = D^-1 A p and xg (the
@@ -160,9 +160,10 @@ static_assert(kSlotWords == 32 * kPacketWords, "a packet for every lane");
 // size (up to one); hop 1 goes to every CTA of the own group, hop 2 from a
 // member of each group to the members of the same rank elsewhere.  kLocal: the
 // CTAs are one cluster, one group, and the packets go to the readers' shared
-// memory.  An iteration on 48 tiles (12 CTAs) takes 3.83 us that way and 4.27 us
-// with packets through L2, on 8 tiles 3.62 and 4.04; 16 CTAs is the largest
-// cluster, and with four tiles each it holds boxes of up to 64.
+// memory.  That took an iteration on 48 tiles (12 CTAs) from 4.27 us with
+// packets through L2 to 3.83, on 8 tiles from 4.04 to 3.62 (3.26 us on 48 tiles
+// with the scalars taken once); 16 CTAs is the largest cluster, and with four
+// tiles each it holds boxes of up to 64.
 constexpr uint32_t kClusterMax = 16;
 constexpr uint32_t kLocalWords = 2 * kClusterMax * 2 * kSums;  // [2][sender][two words of a sum]
 template <bool kLocal>
