@@ -484,9 +484,15 @@ __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_ids_kernel(
     if (kNodes > 1 && total <= kIdList) {
         if (lane < count) {
             const uint32_t b = b0 + lane;
+            const uint32_t* from = masks + (size_t)b * 16u;
             uint4 m[4];
+            if ((reinterpret_cast<uintptr_t>(masks) & 15u) == 0u) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) m[k] = reinterpret_cast<const uint4*>(masks + (size_t)b * 16u)[k];
+                for (int k = 0; k < 4; ++k) m[k] = reinterpret_cast<const uint4*>(from)[k];
+            } else {  // a caller's pointer into a larger buffer
+#pragma unroll
+                for (int k = 0; k < 4; ++k) m[k] = make_uint4(from[4 * k], from[4 * k + 1], from[4 * k + 2], from[4 * k + 3]);
+            }
             uint16_t* at = list + ((lane ? node_voxels[b - 1u] : start) - start);
             const RefSolid sol = ref_solid(keys[b], g);
 #pragma unroll
