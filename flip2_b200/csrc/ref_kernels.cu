@@ -988,26 +988,30 @@ __global__ void __launch_bounds__(kNodeThreads) ref_gs_kernel(
 // ones that move (no apron, no solid), in registers with
 //   p' = (1 - w) p + w (c - D / Adg), c = (scale / Adg) * sum of the coupled neighbours' p,
 // the neighbours summed as a tree: 7 dependent operations instead of 12 and a
-// division.  At y = 0 and y = 7 the index v -+ 8 reaches a voxel of the same
-// color in the next plane; it is read as the last iteration left it, from a
-// copy.  The residual that the reference reads is that of the last sweep,
-// taken by its own formula.  160 nodes: 1.76 us per iteration by
-// ref_gs_kernel, 0.48 us here.
+// division.  The residual that the reference reads is that of the last sweep,
+// taken by its own formula.  160 nodes: 1.78 us per iteration by
+// ref_gs_kernel, 0.35 us here.
+// The apron test lets y = 0 and y = 7 move, where the index v -+ 8 names a
+// voxel of the same color in the next plane, with y = 7 or 0.  No sweep reads
+// one: a particle marks no voxel of the plane y = 0 (its stencil coordinate
+// is at least 2, and the column two below it is never nearer than the radius),
+// so a listed voxel there is a solid one, which neither moves nor is coupled,
+// and one that is not listed has D = 0.  The order within a color is then free.
 constexpr int kSorThreads = 160;  // 144 voxels of a color can move
 __global__ void __launch_bounds__(kSorThreads) ref_gs_long_kernel(
     uint32_t nodes, const uint32_t* __restrict__ node_voxels, const uint32_t* __restrict__ voxel_ids,
     const int8_t* __restrict__ solids, const double* __restrict__ divU, double* __restrict__ p, double* __restrict__ res,
     double scale, double w, uint32_t iters) {
-    __shared__ double D[512], P[512], Q[2][512], Rr[512];
+    __shared__ double D[512], P[512], Rr[512];
     __shared__ int8_t S[512], in[512];
     const uint32_t b = blockIdx.x, tid = threadIdx.x;
-    for (int i = tid; i < 512; i += kSorThreads) { D[i] = 0.0; P[i] = Q[0][i] = Q[1][i] = 0.0; Rr[i] = 0.0; S[i] = 0; in[i] = 0; }
+    for (int i = tid; i < 512; i += kSorThreads) { D[i] = 0.0; P[i] = 0.0; Rr[i] = 0.0; S[i] = 0; in[i] = 0; }
     __syncthreads();
     const uint32_t vs = b ? node_voxels[b - 1] : 0u, ve = node_voxels[b];
     for (uint32_t k = vs + tid; k < ve; k += kSorThreads) {
         const uint32_t id = voxel_ids[k];
         D[id] = divU[k];
-        P[id] = Q[0][id] = Q[1][id] = p[k];
+        P[id] = p[k];
         S[id] = solids[k];
         in[id] = 1;
     }
@@ -1015,7 +1019,7 @@ __global__ void __launch_bounds__(kSorThreads) ref_gs_long_kernel(
     // color 1 (red: even x + y + z) goes first
     const int step[6] = {-1, 1, -8, 8, -64, 64};
     int v[2];
-    bool move[2], wrap_lo[2], wrap_hi[2], couple[2][6];
+    bool move[2], couple[2][6];
     double Adg[2], own[2], coef[2], base[2], pv[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -1023,8 +1027,6 @@ __global__ void __launch_bounds__(kSorThreads) ref_gs_long_kernel(
         const int x = 1 + 2 * x3 + ((1 + y + z + c) & 1);  // c = 0: red, even parity
         v[c] = tid < 144u ? x + 8 * y + 64 * z : 73;
         move[c] = tid < 144u && in[v[c]] && !S[v[c]];
-        wrap_lo[c] = y == 0;
-        wrap_hi[c] = y == 7;
         double Ad = 0.0;
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
@@ -1039,18 +1041,13 @@ __global__ void __launch_bounds__(kSorThreads) ref_gs_long_kernel(
         pv[c] = P[v[c]];
     }
     for (uint32_t it = 0; it < iters; ++it) {
-        const double* last = Q[(it & 1u) ^ 1u];
-        double* now = Q[it & 1u];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             if (move[c]) {
                 const int i = v[c];
                 double n[6];
 #pragma unroll
-                for (int k = 0; k < 6; ++k) {
-                    const double* from = (k == 2 && wrap_lo[c]) || (k == 3 && wrap_hi[c]) ? last : P;
-                    n[k] = couple[c][k] ? from[i + step[k]] : 0.0;
-                }
+                for (int k = 0; k < 6; ++k) n[k] = couple[c][k] ? P[i + step[k]] : 0.0;
                 const double sum = ((n[0] + n[1]) + (n[2] + n[3])) + (n[4] + n[5]);
                 const double pn = fma(coef[c], sum, fma(own[c], pv[c], base[c]));
                 if (it + 1u == iters && c == 1) {  // the last sweep's residual (red's is written as 0)
@@ -1061,7 +1058,6 @@ __global__ void __launch_bounds__(kSorThreads) ref_gs_long_kernel(
                 }
                 pv[c] = pn;
                 P[i] = pn;
-                if (wrap_lo[c] || wrap_hi[c]) now[i] = pn;
             }
             __syncthreads();
         }
@@ -1271,10 +1267,10 @@ int ref_launch_divergence(uint32_t nodes, const uint32_t* node_voxels, const uin
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-// The solve asks for one iteration, then 1,023, then 1,024 at a time.  Those
-// long chunks end where the sweeps no longer move p; shorter ones (the first
-// iteration, whose residual is read) keep the order in which the list form
-// visits a color.
+// The solve asks for 1 and 1,023 iterations in turn (fewer at its cap) and
+// reads the residual after the single ones, which stay with the list form and
+// its order of operations.  What the long chunks leave in p differs from the
+// list form's by rounding.
 constexpr uint32_t kSorLong = 512;
 int ref_launch_gs(uint32_t nodes, const uint32_t* node_voxels, const uint32_t* voxel_ids, const int8_t* solids,
                   const double* divU, double* p, double* res, double scale, double w, uint32_t iters, cudaStream_t s) {
