@@ -148,6 +148,7 @@ def lib():
         "flip_poisson_generate": (i32, [vp, C.POINTER(PoissonSpec)]),
         "flip_poisson_set": (i32, [vp, vp, vp]),
         "flip_poisson_solve": (i32, [vp, i32, d, i32, C.POINTER(SolveInfo)]),
+        "flip_test_solve_timeout": (i32, [vp, i32, u32, u32]),
         "flip_poisson_read_solution": (i32, [vp, vp]),
         "flip_lp_train_step": (i32, [vp, i32, C.c_float, C.POINTER(d)]),
         "flip_lp_eval": (i32, [vp, vp, vp, vp, C.POINTER(d), i32]),

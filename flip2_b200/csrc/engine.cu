@@ -2394,6 +2394,18 @@ extern "C" int flip_lp_eval(flip_engine* e, const float* r_lin, const float* e_l
     return lp_check_err(e);
 }
 
+extern "C" int flip_test_solve_timeout(flip_engine* e, int which, uint32_t exchange, uint32_t polls) {
+    CHECK_NATIVE("flip_test_solve_timeout");
+    if (which < 0 || which > 2 || (exchange && polls < 1024u))
+        return e->fail(FLIP_ERR_ARG, "flip_test_solve_timeout: bad arguments");
+    E_CUDA(cudaStreamSynchronize(e->stream));
+    free_step_graphs(e);  // the captured steps hold one form of the solve's kernel
+    e->pcg.hook.which = (uint32_t)which;
+    e->pcg.hook.exchange = exchange;
+    e->pcg.hook.polls = polls;
+    return FLIP_OK;
+}
+
 // ------------------------------------------- multilevel preconditioner API
 extern "C" int flip_mg_apply(flip_engine* e, const float* r_lin, float* z_lin) {
     CHECK_NATIVE("flip_mg_apply");

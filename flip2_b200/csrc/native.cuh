@@ -46,6 +46,13 @@ constexpr int kResidentNoFar = 29;  // tiles a CTA whose faces always have room 
 constexpr int kResidentMaxCtas = 160;
 constexpr int kPcgSlotWords = 512;
 
+// Test hook of the resident solve's bounded waits: from exchange `exchange` on
+// (from 1; 0: no hook) the last CTA's wait of kind `which` (0, 1: hop 1 and 2 of
+// the sums, 2: face cells) has nothing to end it but the limit of `polls`.
+struct ResidentHook {
+    uint32_t which = 0, exchange = 0, polls = 0;
+};
+
 // PCG vectors on the tile-blocked slots.  The solution is x + xg: x in FP64
 // holds everything up to the last true-residual check, xg (FP32) the
 // increments since then.  An FP32 solution alone bounds the attainable true
@@ -67,6 +74,7 @@ struct PcgBuffers {
     bool cluster;      // ... and they run as one cluster (nat_pcg_cluster)
     unsigned long long* slots;  // its packets, [2][2][ctas][kPcgSlotWords]
     uint32_t* epoch;   // the last tag the resident solve used
+    ResidentHook hook;
     float* far;        // its faces without room on the chip: 768 floats a tile
     unsigned long long* mail;  // its mailboxes: [2][mail_tiles][6][64] tagged words
     uint32_t mail_tiles;

@@ -148,6 +148,7 @@ struct Args {
     uint32_t* epoch;          // the last tag of the solve before
     uint32_t* err;
     int chunk, limit;
+    ResidentHook hook;
 };
 __device__ __forceinline__ unsigned long long tagged(uint32_t tag, uint32_t v) { return ((unsigned long long)tag << 32) | v; }
 
@@ -166,7 +167,9 @@ static_assert(kSlotWords == 32 * kPacketWords, "a packet for every lane");
 // tiles each it holds boxes of up to 64.
 constexpr uint32_t kClusterMax = 16;
 constexpr uint32_t kLocalWords = 2 * kClusterMax * 2 * kSums;  // [2][sender][two words of a sum]
-template <bool kLocal>
+// kHook: with the test hook (kernels of their own: the checks in the polling
+// loops cost 0.5 us an iteration on 392 tiles).
+template <bool kLocal, bool kHook>
 struct Exchange {
     unsigned long long* slots;
     uint32_t local;   // kLocal: the packets' address in shared memory
@@ -175,7 +178,10 @@ struct Exchange {
     uint32_t tag;     // number of the exchange in flight; its low bit picks the half
     uint32_t n;       // CTAs taking part
     uint32_t groups, group, first, size, rank;  // group's first CTA, its size, the own rank in it
+    uint32_t hook_which, hook_tag, hook_polls;  // kHook: in force from that tag on
 
+    __device__ __forceinline__ bool in_vain(uint32_t which) const { return kHook && which == hook_which && tag >= hook_tag; }
+    __device__ __forceinline__ uint32_t polls() const { return kHook ? hook_polls : kSpin; }
     __device__ __forceinline__ uint32_t group_first(uint32_t g) const { return g * n / groups; }
     __device__ __forceinline__ void init(uint32_t count) {
         n = count;
@@ -216,7 +222,7 @@ struct Exchange {
         uint32_t spin = 0;
         bool ok;
         do {
-            ok = true;
+            ok = !in_vain(hop);
 #pragma unroll
             for (int k = 0; k < kSums; ++k) {
                 if (kLocal) ld_cluster_u64x2(l + 16u * k, u[2 * k], u[2 * k + 1]);
@@ -225,7 +231,7 @@ struct Exchange {
 #pragma unroll
             for (int k = 0; k < 2 * kSums; ++k) ok = ok && (uint32_t)(u[k] >> 32) == tag;
             ok = __all_sync(0xffffffffu, ok);
-        } while (!ok && ++spin < kSpin);
+        } while (!ok && ++spin < polls());
 #pragma unroll
         for (int k = 0; k < kSums; ++k)
             v[k] = lane < count ? __longlong_as_double((long long)((u[2 * k + 1] << 32) | (uint32_t)u[2 * k])) : 0.0;
@@ -269,7 +275,7 @@ struct Exchange {
             bool ok = poll(0, lane, size, w);
             asm volatile("bar.arrive 1, 512;" ::: "memory");
             lanes_sum(w, lane);
-            if (!kLocal && groups > 1) {
+            if (!kLocal && groups > 1 && ok) {  // a group that misses a packet has no sums to pass on
                 if (kFence) __threadfence();
                 if (lane < (int)groups) {
                     // a CTA of rank r hears from rank r modulo the group's size (in its own group: itself)
@@ -277,7 +283,7 @@ struct Exchange {
                     for (uint32_t r = rank; r < s2; r += size) push(1, f2 + r, group, w);
                 }
                 __syncwarp();
-                ok = poll(1, lane, groups, w) && ok;
+                ok = poll(1, lane, groups, w);
                 lanes_sum(w, lane);
             }
             if (kFence) __threadfence();
@@ -307,8 +313,8 @@ struct Plan {
 // The solve on one CTA's tiles.  kAll: w, t and xg in shared memory; else w
 // in registers for kReg passes, then in shared memory as far as it fits, and
 // t and xg in global memory.
-template <int kReg, bool kAll, bool kLocal>
-__device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* pool, Exchange<kLocal> X, const Plan P) {
+template <int kReg, bool kAll, bool kLocal, bool kHook>
+__device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* pool, Exchange<kLocal, kHook> X, const Plan P) {
     const int tid = threadIdx.x, g = tid >> 7, u = tid & 127;
     const int row = u >> 1, half = u & 1, cy = row & 7, cz = row >> 3, cx = 4 * half;
     const uint32_t lo = (uint32_t)(cx + 8 * row), cnt = P.cnt;
@@ -438,8 +444,9 @@ __device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* p
     auto fetch_mail = [&](uint32_t e, unsigned long long (&v)[4]) {  // until the warp's are there
         uint32_t spin = 0;
         while (!__all_sync(0xffffffffu, (uint32_t)(v[0] >> 32) == X.tag && (uint32_t)(v[1] >> 32) == X.tag &&
-                                            (uint32_t)(v[2] >> 32) == X.tag && (uint32_t)(v[3] >> 32) == X.tag)) {
-            if (++spin >= kSpin) { S.lost = 1; break; }
+                                            (uint32_t)(v[2] >> 32) == X.tag && (uint32_t)(v[3] >> 32) == X.tag &&
+                                            !X.in_vain(2))) {
+            if (++spin >= X.polls()) { S.lost = 1; break; }
             load_mail(e, v);
         }
     };
@@ -723,14 +730,14 @@ __device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* p
 }
 
 // kLocal: one cluster of at most kClusterMax CTAs, four tiles each
-template <bool kLocal>
+template <bool kLocal, bool kHook>
 __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_constant__ Args A, const uint32_t* __restrict__ d_ntiles) {
     extern __shared__ __align__(16) unsigned char smem[];
     Fixed& S = *reinterpret_cast<Fixed*>(smem);
     float* pool = reinterpret_cast<float*>(smem + sizeof(Fixed));
     const uint32_t nt = *d_ntiles;
     if (A.st->done || nt > (uint32_t)kMaxTiles * A.ctas) return;  // solved already, or more than the chip holds
-    Exchange<kLocal> X;
+    Exchange<kLocal, kHook> X;
     const uint32_t ctas = min(A.ctas, (nt + kGroups - 1u) / kGroups);
     if (blockIdx.x >= ctas) return;
     X.init(ctas);
@@ -738,6 +745,11 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     X.ctas = A.ctas;
     X.S = &S;
     X.tag = *A.epoch;
+    if (kHook) {
+        X.hook_which = blockIdx.x == ctas - 1u ? A.hook.which : 3u;
+        X.hook_tag = X.tag + A.hook.exchange;
+        X.hook_polls = A.hook.polls;
+    }
     Plan P;
     P.t0 = (uint32_t)((uint64_t)nt * blockIdx.x / X.n);
     P.cnt = (uint32_t)((uint64_t)nt * (blockIdx.x + 1) / X.n) - P.t0;
@@ -822,7 +834,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         P.off_x = P.off_t + 512u * cnt;
         P.n_w = cnt;
         P.n_face_w = P.nface;
-        resident_solve<0, true, kLocal>(A, S, pool, X, P);
+        resident_solve<0, true, kLocal, kHook>(A, S, pool, X, P);
     } else if (!kLocal) {
         const uint32_t faces = min(P.nface, room);
         P.off_w = base + 64u * faces;
@@ -830,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
         P.face_w = P.off_w + 512u * P.n_w;
         P.n_face_w = min(P.nface, (left - 64u * faces - 512u * P.n_w) / 64u);
         P.off_t = P.off_x = 0;
-        resident_solve<kRegPasses, false, kLocal>(A, S, pool, X, P);
+        resident_solve<kRegPasses, false, kLocal, kHook>(A, S, pool, X, P);
     }
     if (kLocal) cluster_sync();  // no CTA leaves while another may still write to it
 }
@@ -867,12 +879,13 @@ cudaLaunchConfig_t resident_config(uint32_t grid, cudaLaunchAttribute* attr, boo
 int nat_pcg_cluster(uint32_t ctas, bool* fits) {
     *fits = false;
     if (ctas > kClusterMax) return FLIP_OK;
-    FLIP_CUDA_TRY(cudaFuncSetAttribute(pcg_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
-    FLIP_CUDA_TRY(cudaFuncSetAttribute(pcg_resident_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    const auto kernel = pcg_resident_kernel<true, false>;
+    FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = resident_config(cluster_of(ctas), attr, true, nullptr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, pcg_resident_kernel<true>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();  // no such cluster on this device
         return FLIP_OK;
     }
@@ -882,12 +895,15 @@ int nat_pcg_cluster(uint32_t ctas, bool* fits) {
 
 int nat_launch_pcg_resident(const uint32_t* tiles, const uint32_t* d_ntiles, const NatDims& D, PcgBuffers& B, int chunk,
                             int limit, uint32_t* err, cudaStream_t s) {
-    const auto kernel = B.cluster ? pcg_resident_kernel<true> : pcg_resident_kernel<false>;
+    const bool hook = B.hook.exchange != 0;
+    const auto kernel = B.cluster ? (hook ? pcg_resident_kernel<true, true> : pcg_resident_kernel<true, false>)
+                                  : (hook ? pcg_resident_kernel<false, true> : pcg_resident_kernel<false, false>);
+    if (B.cluster && hook) FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = resident_config(B.cluster ? cluster_of(B.ctas) : B.ctas, attr, B.cluster, s);
     const Args A{tiles, B.tcoord, D, B.x, B.xg, B.r, B.q, B.far, B.mail, 64u * 6u * B.mail_tiles, B.b, B.cell, B.st, B.slots,
-                 B.ctas, B.epoch, err, chunk, limit};
+                 B.ctas, B.epoch, err, chunk, limit, B.hook};
     FLIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A, d_ntiles));
     return FLIP_OK;
 }

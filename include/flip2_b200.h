@@ -366,6 +366,15 @@ int flip_get_solve_info(flip_engine* e, flip_solve_info* out);
  * coarsest solve).  Methods 1 and 2 restart Jacobi-PCG from x = 0 when they
  * miss tol within max_iter or stall. */
 int flip_poisson_solve(flip_engine* e, int method, double tol, int max_iter, flip_solve_info* info);
+/* Test hook for the bounded waits of the Jacobi-PCG solve that runs as one
+ * resident kernel (no reference counterpart): in every such solve of the engine
+ * from here on, captured ones included, the last CTA waits from exchange number
+ * `exchange` on (counted from 1; 0: hook off) for a word that nothing publishes
+ * -- which = 0: the sums of its group of CTAs, 1: those of the other groups
+ * (with more than 32 CTAs), 2: the face cells of a neighbouring CTA -- and every
+ * wait gives up after `polls` polls (1,024 at least) instead of about two
+ * seconds.  The solve then ends with FLIP_ERR_TIMEOUT and bit 4 of error_flags. */
+int flip_test_solve_timeout(flip_engine* e, int which, uint32_t exchange, uint32_t polls);
 /* solution (FP64) in x-fastest order */
 int flip_poisson_read_solution(flip_engine* e, double* x_lin);
 /* The solver applies M(r) = N(r) + D^-1 r (network plus Jacobi).  One
