@@ -597,7 +597,9 @@ __device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* p
             }, [&](const double (&w)[kSums], int lane) {
                 // ---- scalars, once for the CTA (every thread dividing for itself
                 // took 3.81 instead of 3.26 us an iteration on 48 tiles); a verdict of
-                // 1: the residual before this step claims convergence
+                // 1: the residual before this step claims convergence.  Not before the
+                // first one: what a start may claim, nat_launch_pcgw_init has settled,
+                // and r.r = b.b <= tol^2 b.b also where both are infinite
                 const double a = w[3] / w[0], over = 1.0 / w[3];
                 const double b = fmax(fma(a, fma(a, w[2], -2.0 * w[1]), w[3]), 0.0) * over;
                 if (lane == 0) {
@@ -606,7 +608,7 @@ __device__ __forceinline__ void resident_solve(const Args& A, Fixed& S, float* p
                     S.rz = w[3];
                     S.alpha = (float)a;
                     S.beta = (float)b;
-                    S.verdict = w[4] <= stop ? 1u : (w[0] > 0.0 ? 0u : 2u);
+                    S.verdict = iter > 0 && w[4] <= stop ? 1u : (w[0] > 0.0 ? 0u : 2u);
                 }
             })) { lost = true; break; }
         const bool pending = S.verdict == 1u;
