@@ -823,9 +823,13 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_resident_kernel(const __grid_
     }
     __syncthreads();
     P.nface = S.nface;
-    // Everything on the chip where the largest share of tiles with six faces
-    // each would fit (the same branch in every CTA): 22 tiles a CTA.  Else w in
-    // what the registers and the pool hold, then the faces' w.
+    // Everything on the chip where the largest share of tiles has room for it with
+    // three faces a tile towards other CTAs (21 tiles) and this CTA's own faces
+    // have; else w in what the registers and the pool hold, then the faces' w.
+    // The second condition is the CTA's own: both forms take the same exchanges,
+    // publish the same face cells and leave the same xg and r for a check, so CTAs
+    // of either form work together (21 tiles each in rows of 22: 50 of 148 keep
+    // everything on the chip).
     const uint32_t most = (nt + X.n - 1u) / X.n;
     const uint32_t left = (uint32_t)kPoolFloats - base;
     if (kLocal) cluster_sync();  // every CTA's packets are ready
