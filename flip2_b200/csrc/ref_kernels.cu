@@ -465,66 +465,101 @@ __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_giants_kernel(
 }
 
 // generateVoxelIDs (particles.cu:192-321): compaction from the masks.  A warp
-// takes 32 nodes: each lane lists its node's voxels into shared memory, and
-// the warp copies the list out in order.  Nodes with more voxels than the list
-// holds, and few nodes (a warp each), are written straight from their masks,
-// lane l the voxel of bit l of each word.
+// lists the voxels of kNodes nodes in shared memory, 32 / kNodes lanes a node,
+// and copies the list out in order.  Bound by the lanes' walks over their words'
+// bits: eight lanes a node have the shortest, a lane a node takes the fewest
+// instructions, which pays where nodes are many and sparse (the launch says
+// from where); nodes too dense for its list then go in fours.  Four nodes with
+// more voxels than the list holds are written straight from their masks, lane l
+// the voxel of bit l of each word.
 constexpr uint32_t kIdList = 1280;
+// nodes b0 .. b0 + count - 1, `total` voxels from `start` on
+template <int kNodes>
+__device__ __forceinline__ void ref_list_ids(uint32_t b0, uint32_t count, uint32_t start, uint32_t total,
+                                             const uint32_t* __restrict__ keys, const uint32_t* __restrict__ masks,
+                                             const uint32_t* __restrict__ node_voxels, const flip_grid& g, uint16_t* list,
+                                             uint32_t* __restrict__ voxel_ids, int8_t* __restrict__ solids) {
+    constexpr uint32_t kLanes = 32 / kNodes, kWords = kNodes == 32 ? 16 : 16 / kLanes;  // lanes a node, words a lane
+    const uint32_t lane = threadIdx.x & 31u, b = b0 + lane / kLanes;
+    const bool have = lane / kLanes < count;
+    uint32_t m[kWords], at = 0;
+    if (have) {
+        const uint32_t* from = masks + (size_t)b * 16u + (lane % kLanes) * kWords;
+        if (kWords % 4 == 0 && (reinterpret_cast<uintptr_t>(masks) & 15u) == 0u) {
+#pragma unroll
+            for (uint32_t k = 0; k + 4u <= kWords; k += 4u) {
+                const uint4 q = *reinterpret_cast<const uint4*>(from + k);
+                m[k] = q.x; m[k + 1] = q.y; m[k + 2] = q.z; m[k + 3] = q.w;
+            }
+        } else {  // (also a caller's pointer into a larger buffer)
+#pragma unroll
+            for (uint32_t k = 0; k < kWords; ++k) m[k] = from[k];
+        }
+        if (kNodes == 32 && lane) at = node_voxels[b - 1u] - start;
+    }
+    if (kNodes < 32) {
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kWords; ++k) n += have ? __popc(m[k]) : 0u;
+        at = warp_inclusive_scan(n) - n;
+    }
+    if (have) {
+        const RefSolid sol = ref_solid(keys[b], g);
+        uint16_t* to = list + at;
+#pragma unroll
+        for (uint32_t k = 0; k < kWords; ++k)
+            for (uint32_t word = m[k]; word; word &= word - 1u) {
+                const uint32_t id = 32u * (kWords * (lane % kLanes) + k) + (uint32_t)__ffs(word) - 1u;
+                *to++ = (uint16_t)(id | (sol.at(id) << 15));  // bit 15: solid
+            }
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < total; i += 32u) {
+        const uint32_t v = list[i];
+        voxel_ids[start + i] = v & 511u;
+        solids[start + i] = (int8_t)(v >> 15);
+    }
+    __syncwarp();  // the list is free
+}
 template <int kNodes>
 __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_ids_kernel(
     const uint32_t* __restrict__ keys, uint32_t nodes, const uint32_t* __restrict__ masks,
     const uint32_t* __restrict__ node_voxels, flip_grid g, uint32_t* __restrict__ voxel_ids, int8_t* __restrict__ solids) {
-    __shared__ uint16_t lists[kVoxWarps][kNodes > 1 ? kIdList : 1];  // bit 15: solid
+    __shared__ uint16_t lists[kVoxWarps][kIdList];
     uint16_t* list = lists[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t b0 = (blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kNodes;
-    if (b0 >= nodes) return;
-    const uint32_t count = min((uint32_t)kNodes, nodes - b0);
-    const uint32_t start = b0 ? node_voxels[b0 - 1u] : 0u, total = node_voxels[b0 + count - 1u] - start;
-    if (kNodes > 1 && total <= kIdList) {
-        if (lane < count) {
-            const uint32_t b = b0 + lane;
-            const uint32_t* from = masks + (size_t)b * 16u;
-            uint4 m[4];
-            if ((reinterpret_cast<uintptr_t>(masks) & 15u) == 0u) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) m[k] = reinterpret_cast<const uint4*>(from)[k];
-            } else {  // a caller's pointer into a larger buffer
-#pragma unroll
-                for (int k = 0; k < 4; ++k) m[k] = make_uint4(from[4 * k], from[4 * k + 1], from[4 * k + 2], from[4 * k + 3]);
-            }
-            uint16_t* at = list + ((lane ? node_voxels[b - 1u] : start) - start);
-            const RefSolid sol = ref_solid(keys[b], g);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                for (uint32_t word = (&m[k >> 2].x)[k & 3]; word; word &= word - 1u) {
-                    const uint32_t id = 32u * k + (uint32_t)__ffs(word) - 1u;
-                    *at++ = (uint16_t)(id | (sol.at(id) << 15));
-                }
+    const uint32_t first = (blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kNodes;
+    if (first >= nodes) return;
+    const uint32_t last = min(first + kNodes, nodes);
+    auto end_of = [&](uint32_t b) { return b ? node_voxels[b - 1u] : 0u; };  // of the nodes before b
+    if (kNodes == 32) {
+        const uint32_t start = end_of(first), total = end_of(last) - start;
+        if (total <= kIdList) {
+            ref_list_ids<kNodes>(first, last - first, start, total, keys, masks, node_voxels, g, list, voxel_ids, solids);
+            return;
         }
-        __syncwarp();
-        for (uint32_t i = lane; i < total; i += 32u) {
-            const uint32_t v = list[i];
-            voxel_ids[start + i] = v & 511u;
-            solids[start + i] = (int8_t)(v >> 15);
-        }
-        return;
     }
-    for (uint32_t r = 0; r < count; ++r) {
-        const uint32_t b = b0 + r;
-        const uint32_t m = lane < 16u ? masks[(size_t)b * 16u + lane] : 0u;
-        uint32_t at = b ? node_voxels[b - 1u] : 0u;
-        const RefSolid sol = ref_solid(keys[b], g);
-        // the mask words that hold a voxel, in order
-        for (uint32_t rest = __ballot_sync(0xffffffffu, m != 0u); rest; rest &= rest - 1u) {
-            const int q = __ffs(rest) - 1;
-            const uint32_t word = __shfl_sync(0xffffffffu, m, q);
-            if ((word >> lane) & 1u) {
-                const uint32_t i = (uint32_t)q * 32u + lane, pos = at + __popc(word & ((1u << lane) - 1u));
-                voxel_ids[pos] = i;
-                solids[pos] = (int8_t)sol.at(i);
+    for (uint32_t b0 = first; b0 < last; b0 += 4u) {
+        const uint32_t count = min(4u, last - b0), start = end_of(b0), total = end_of(b0 + count) - start;
+        if (total <= kIdList) {
+            ref_list_ids<4>(b0, count, start, total, keys, masks, node_voxels, g, list, voxel_ids, solids);
+            continue;
+        }
+        for (uint32_t b = b0; b < b0 + count; ++b) {
+            const uint32_t m = lane < 16u ? masks[(size_t)b * 16u + lane] : 0u;
+            uint32_t at = end_of(b);
+            const RefSolid sol = ref_solid(keys[b], g);
+            // the mask words that hold a voxel, in order
+            for (uint32_t rest = __ballot_sync(0xffffffffu, m != 0u); rest; rest &= rest - 1u) {
+                const int q = __ffs(rest) - 1;
+                const uint32_t word = __shfl_sync(0xffffffffu, m, q);
+                if ((word >> lane) & 1u) {
+                    const uint32_t i = (uint32_t)q * 32u + lane, pos = at + __popc(word & ((1u << lane) - 1u));
+                    voxel_ids[pos] = i;
+                    solids[pos] = (int8_t)sol.at(i);
+                }
+                at += __popc(word);
             }
-            at += __popc(word);
         }
     }
 }
@@ -1209,11 +1244,17 @@ int ref_launch_voxel_counts(const uint32_t* starts, const uint32_t* keys, uint32
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
+// Ids: 32 nodes a warp from this many on.  Four a warp and 32 a warp, nodes with
+// some 27 voxels each: 165,000 31 and 50 us, 524,000 74 and 71, 2.6 million 359 and
+// 256; with 60 and more voxels (32 lists in fours then) 258,000 57 and 72, 982,000
+// 187 and 210, 4 million 715 and 773.  A warp a node takes 56, 170, 738 and 109, 383,
+// 1,534 us, and is no faster from 300 nodes on (15 us both).
+constexpr uint32_t kManyNodes = 1u << 19;
 int ref_launch_voxel_ids(const uint32_t* keys, uint32_t nodes, const uint32_t* masks, const uint32_t* node_voxels,
                          const flip_grid& g, uint32_t* voxel_ids, int8_t* solids, cudaStream_t s) {
     if (!nodes) return FLIP_OK;
-    const uint32_t per = (nodes >= kSparseNodes ? 32u : 1u) * kVoxWarps, grid = (nodes + per - 1) / per;
-    const auto kernel = nodes >= kSparseNodes ? ref_voxel_ids_kernel<32> : ref_voxel_ids_kernel<1>;
+    const uint32_t per = (nodes >= kManyNodes ? 32u : 4u) * kVoxWarps, grid = (nodes + per - 1) / per;
+    const auto kernel = nodes >= kManyNodes ? ref_voxel_ids_kernel<32> : ref_voxel_ids_kernel<4>;
     kernel<<<grid, 32 * kVoxWarps, 0, s>>>(keys, nodes, masks, node_voxels, g, voxel_ids, solids);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
