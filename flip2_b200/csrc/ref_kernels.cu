@@ -306,8 +306,13 @@ __device__ __forceinline__ RefSolid ref_solid(uint32_t key, const flip_grid& g) 
 // its solid voxels here and the others from ref_voxel_giants_kernel: left to
 // one warp, such nodes were 25 of 38 ms at 64M particles.
 constexpr int kVoxWarps = 8;
-constexpr uint32_t kVoxLong = 8;      // particles above which the warp takes a sparse variant's node together
-constexpr uint32_t kVoxGiant = 1024;  // ... and above which several warps do
+// Particles above which the warp takes a sparse variant's node together: at 4, 8,
+// 16 and never, 24 million nodes of 2.5 took 3.27, 2.35, 2.37 and 2.38 ms, and with a
+// tenth of the positions clamped to the faces 2.51, 2.46, 2.47 and 8.63 ms.
+constexpr uint32_t kVoxLong = 8;
+// ... and above which several warps do: at 256, 1,024 and 4,096, 59 million
+// particles took 2.47, 2.35 and 2.31 ms, clamped ones 2.56, 2.46 and 3.82 ms.
+constexpr uint32_t kVoxGiant = 1024;
 struct VoxWarp {
     unsigned long long planes[8 * kVoxStride];
     uint32_t mask[32 * 17];  // rows of 16 words, padded: the masks of the warp's nodes
@@ -1218,11 +1223,18 @@ int ref_launch_ydim(const uint32_t* starts, const uint32_t* keys, uint32_t nodes
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-// A lane a node where that makes warps for every SM (65,536 nodes: 14 a SM)
-// and a node holds few particles (below 8 a warp's lanes differ little); 8
-// lanes a node for fewer such nodes, a warp a node for dense ones.  The pass
-// over the giants pays its launch from kVoxGiantFrom particles.
-constexpr uint32_t kSparseNodes = 65536;
+// Lanes a node, in us for 1, 8 and 32.  Below 8 particles a node a lane is
+// enough once there are warps for every SM (4 particles: 32,000 nodes 22, 22 and
+// 38, 63,000 25, 30 and 65, 257,000 50, 82 and 229; at 8, 262,000 124, 106 and
+// 244).  Eight lanes wait less for the fullest node than a warp idles over the
+// others', up to some 128 particles a node and where nodes fill the chip (16,000
+// nodes of 8, 64, 128, 315 particles: 19 and 25, 35 and 37, 54 and 50, 126 and 99;
+// 64,000: 35 and 66, 97 and 123, 160 and 181, 347 and 348); a warp a node keeps
+// fewer, denser ones (4,096 nodes of 64, 315: 21 and 20, 50 and 35).
+constexpr uint32_t kSparseNodes = 65536, kWideNodes = 16384;
+constexpr uint64_t kSparsePer = 8, kWidePer = 128;
+// The pass over the giants takes 3 to 5 us (32,768 particles: 19.7 with it, 15.8
+// without); a warp by itself takes 25 us for each 1,024 particles of a node.
 constexpr uint64_t kVoxGiantFrom = 32768;
 int ref_launch_voxel_counts(const uint32_t* starts, const uint32_t* keys, uint32_t nodes, uint64_t n, const double* px,
                             const double* py, const double* pz, const flip_grid& g, uint32_t* counts, uint32_t* masks,
@@ -1232,7 +1244,8 @@ int ref_launch_voxel_counts(const uint32_t* starts, const uint32_t* keys, uint32
     static_assert(sizeof(VoxWarp) * kVoxWarps <= 49152, "within the default shared memory");
     const bool giants = n > kVoxGiantFrom;
     const uint32_t giant = giants ? kVoxGiant : 0xFFFFFFFFu;
-    const int lanes = n < 8ull * nodes ? (nodes >= kSparseNodes ? 1 : 8) : 32;
+    const int lanes = n < kSparsePer * nodes ? (nodes >= kSparseNodes ? 1 : 8)
+                                             : (nodes >= kWideNodes && n < kWidePer * nodes ? 8 : 32);
     const uint32_t per = 32u / (uint32_t)lanes * kVoxWarps, grid = (nodes + per - 1) / per;
     const auto kernel = lanes == 1 ? ref_voxel_counts_kernel<1> : (lanes == 8 ? ref_voxel_counts_kernel<8> : ref_voxel_counts_kernel<32>);
     kernel<<<grid, 32 * kVoxWarps, smem, s>>>(starts, keys, nodes, n, px, py, pz, g, giant, counts, masks);
@@ -1259,7 +1272,10 @@ int ref_launch_voxel_ids(const uint32_t* keys, uint32_t nodes, const uint32_t* m
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-// cells from this many particles a node on average
+// Cells from this many particles a node on average: the two forms cross at 16
+// to 24 (scatter and cells, 4,096 nodes of 8, 16, 32, 64 particles: 328 and 352, 390
+// and 363, 463 and 379, 529 and 437 us; 27,000 of 8, 16, 24, 32: 1,829 and 2,179, 2,233
+// and 2,259, 2,499 and 2,302, 2,687 and 2,337), with a few hundred nodes earlier.
 constexpr uint64_t kP2gDense = 32;
 int ref_launch_p2g(const uint32_t* starts, const uint32_t* keys, uint32_t nodes, uint64_t n, const double* px,
                    const double* py, const double* pz, const double* vx, const double* vy, const double* vz,

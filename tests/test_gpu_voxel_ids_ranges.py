@@ -1,8 +1,8 @@
-"""The compaction of voxel ids (generateVoxelIDs, particles.cu:192-321) on both
-sides of its lines, bit-exact against the oracle: four nodes a warp and 32 a
-warp (524,288 nodes and more), warps whose nodes have more voxels than a list
-holds and warps whose nodes have not, four nodes that do not fit one either,
-and a last warp with nodes missing."""
+"""Voxel counts by eight lanes a node in dense boxes, and the compaction of
+voxel ids on both sides of its lines (particles.cu:88-321), bit-exact against the
+oracle: four nodes a warp and 32 a warp (524,288 nodes and more), warps whose
+nodes have more voxels than a list holds and warps whose nodes have not, four
+nodes that do not fit one either, and a last warp with nodes missing."""
 import numpy as np
 import pytest
 
@@ -24,6 +24,8 @@ CASES = {
     "one node": (3, (4, 4, 4), 0.0),
     "dense": (12001, (7, 6, 5), 0.0),
     "sparse": (30017, (60, 61, 62), 0.0),
+    "eight lanes, dense": (300007, (27, 28, 26), 0.0),
+    "eight lanes, nearly too dense": (2000003, (26, 25, 26), 0.0),
     "many, some of them dense": (1400003, (101, 100, 99), 0.35),
 }
 
@@ -45,6 +47,8 @@ def test_ids_match_the_oracle(name):
         assert (four > LIST).any() and (four <= LIST).any() and b["nodes"] % 4
     if name == "sparse":
         assert b["nodes"] % 4 and b["nodes"] % 32
+    if name.startswith("eight"):
+        assert b["nodes"] >= 16384 and 8 <= n / b["nodes"] < 128
     if name.startswith("many"):
         assert b["nodes"] >= 1 << 19 and b["nodes"] % 32
         assert (all32 > LIST).any() and (all32 <= LIST).any()
