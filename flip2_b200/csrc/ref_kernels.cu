@@ -474,9 +474,9 @@ __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_giants_kernel(
 // and copies the list out in order.  Bound by the lanes' walks over their words'
 // bits: eight lanes a node have the shortest, a lane a node takes the fewest
 // instructions, which pays where nodes are many and sparse (the launch says
-// from where); nodes too dense for its list then go in fours.  Four nodes with
-// more voxels than the list holds are written straight from their masks, lane l
-// the voxel of bit l of each word.
+// from where); nodes too dense for its list then go in fours.  Few nodes (a warp
+// each), and four with more voxels than the list holds, are written straight from
+// their masks, lane l the voxel of bit l of each word.
 constexpr uint32_t kIdList = 1280;
 // nodes b0 .. b0 + count - 1, `total` voxels from `start` on
 template <int kNodes>
@@ -530,14 +530,14 @@ template <int kNodes>
 __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_ids_kernel(
     const uint32_t* __restrict__ keys, uint32_t nodes, const uint32_t* __restrict__ masks,
     const uint32_t* __restrict__ node_voxels, flip_grid g, uint32_t* __restrict__ voxel_ids, int8_t* __restrict__ solids) {
-    __shared__ uint16_t lists[kVoxWarps][kIdList];
+    __shared__ uint16_t lists[kVoxWarps][kNodes > 1 ? kIdList : 1];
     uint16_t* list = lists[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = (blockIdx.x * kVoxWarps + (threadIdx.x >> 5)) * kNodes;
     if (first >= nodes) return;
     const uint32_t last = min(first + kNodes, nodes);
     auto end_of = [&](uint32_t b) { return b ? node_voxels[b - 1u] : 0u; };  // of the nodes before b
-    if (kNodes == 32) {
+    if constexpr (kNodes == 32) {
         const uint32_t start = end_of(first), total = end_of(last) - start;
         if (total <= kIdList) {
             ref_list_ids<kNodes>(first, last - first, start, total, keys, masks, node_voxels, g, list, voxel_ids, solids);
@@ -545,10 +545,13 @@ __global__ void __launch_bounds__(32 * kVoxWarps) ref_voxel_ids_kernel(
         }
     }
     for (uint32_t b0 = first; b0 < last; b0 += 4u) {
-        const uint32_t count = min(4u, last - b0), start = end_of(b0), total = end_of(b0 + count) - start;
-        if (total <= kIdList) {
-            ref_list_ids<4>(b0, count, start, total, keys, masks, node_voxels, g, list, voxel_ids, solids);
-            continue;
+        const uint32_t count = min(4u, last - b0);
+        if constexpr (kNodes > 1) {
+            const uint32_t start = end_of(b0), total = end_of(b0 + count) - start;
+            if (total <= kIdList) {
+                ref_list_ids<4>(b0, count, start, total, keys, masks, node_voxels, g, list, voxel_ids, solids);
+                continue;
+            }
         }
         for (uint32_t b = b0; b < b0 + count; ++b) {
             const uint32_t m = lane < 16u ? masks[(size_t)b * 16u + lane] : 0u;
@@ -1257,17 +1260,19 @@ int ref_launch_voxel_counts(const uint32_t* starts, const uint32_t* keys, uint32
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
 }
-// Ids: 32 nodes a warp from this many on.  Four a warp and 32 a warp, nodes with
-// some 27 voxels each: 165,000 31 and 50 us, 524,000 74 and 71, 2.6 million 359 and
-// 256; with 60 and more voxels (32 lists in fours then) 258,000 57 and 72, 982,000
-// 187 and 210, 4 million 715 and 773.  A warp a node takes 56, 170, 738 and 109, 383,
-// 1,534 us, and is no faster from 300 nodes on (15 us both).
-constexpr uint32_t kManyNodes = 1u << 19;
+// Ids: a warp a node below 16,384 nodes, four nodes a warp (512 nodes 11.4 and 15.5
+// us, 15,600 of 200 voxels 17.3 and 16.9, 32,000 of 75 20.9 and 16.6, 79,000 31 and 21,
+// 258,000 109 and 57), and 32 from 524,288 on: with four and 32 a warp, nodes of some 27
+// voxels, 165,000 31 and 50 us, 524,000 74 and 71, 2.6 million 359 and 256; of 60 and more
+// (32 go in fours then) 258,000 57 and 72, 982,000 187 and 210, 4 million 715 and 773,
+// where a warp a node takes 1,534.
+constexpr uint32_t kFewNodes = 16384, kManyNodes = 1u << 19;
 int ref_launch_voxel_ids(const uint32_t* keys, uint32_t nodes, const uint32_t* masks, const uint32_t* node_voxels,
                          const flip_grid& g, uint32_t* voxel_ids, int8_t* solids, cudaStream_t s) {
     if (!nodes) return FLIP_OK;
-    const uint32_t per = (nodes >= kManyNodes ? 32u : 4u) * kVoxWarps, grid = (nodes + per - 1) / per;
-    const auto kernel = nodes >= kManyNodes ? ref_voxel_ids_kernel<32> : ref_voxel_ids_kernel<4>;
+    const uint32_t each = nodes < kFewNodes ? 1u : (nodes < kManyNodes ? 4u : 32u);
+    const uint32_t per = each * kVoxWarps, grid = (nodes + per - 1) / per;
+    const auto kernel = each == 1u ? ref_voxel_ids_kernel<1> : (each == 4u ? ref_voxel_ids_kernel<4> : ref_voxel_ids_kernel<32>);
     kernel<<<grid, 32 * kVoxWarps, 0, s>>>(keys, nodes, masks, node_voxels, g, voxel_ids, solids);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;

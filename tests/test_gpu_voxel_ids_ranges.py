@@ -1,8 +1,9 @@
 """Voxel counts by eight lanes a node in dense boxes, and the compaction of
 voxel ids on both sides of its lines (particles.cu:88-321), bit-exact against the
-oracle: four nodes a warp and 32 a warp (524,288 nodes and more), warps whose
-nodes have more voxels than a list holds and warps whose nodes have not, four
-nodes that do not fit one either, and a last warp with nodes missing."""
+oracle: a warp a node (below 16,384 nodes), four nodes a warp and 32 (524,288
+nodes and more), warps whose nodes have more voxels than a list holds and warps
+whose nodes have not, four nodes that do not fit one either, and a last warp with
+nodes missing."""
 import numpy as np
 import pytest
 
@@ -22,7 +23,8 @@ def groups(b, size):
 CASES = {
     # name: particles, root cells, share of the particles in the box's lowest eighth
     "one node": (3, (4, 4, 4), 0.0),
-    "dense": (12001, (7, 6, 5), 0.0),
+    "dense, a warp a node": (12001, (7, 6, 5), 0.0),
+    "dense, four a warp": (1200001, (28, 26, 27), 0.9),
     "sparse": (30017, (60, 61, 62), 0.0),
     "eight lanes, dense": (300007, (27, 28, 26), 0.0),
     "eight lanes, nearly too dense": (2000003, (26, 25, 26), 0.0),
@@ -43,10 +45,10 @@ def test_ids_match_the_oracle(name):
     pos = u * np.array(size)
     b = O.ref_bin(pos[:, 0].copy(), pos[:, 1].copy(), pos[:, 2].copy(), O.grid(0.0, 0.0, 0.0, *size, 1.0))
     four, all32 = groups(b, 4), groups(b, 32)
-    if name == "dense":
-        assert (four > LIST).any() and (four <= LIST).any() and b["nodes"] % 4
+    if name == "dense, four a warp":
+        assert b["nodes"] >= 16384 and (four > LIST).any() and (four <= LIST).any()
     if name == "sparse":
-        assert b["nodes"] % 4 and b["nodes"] % 32
+        assert b["nodes"] >= 16384 and b["nodes"] % 4
     if name.startswith("eight"):
         assert b["nodes"] >= 16384 and 8 <= n / b["nodes"] < 128
     if name.startswith("many"):
