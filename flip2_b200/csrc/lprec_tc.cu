@@ -26,7 +26,6 @@
 namespace flip {
 
 namespace {
-constexpr int kTcThreads = 256;   // 8 warps: 2 warpgroups for the TMEM reads
 constexpr int kTcCols = 128;      // 8 z-slices x 16 FP32 columns
 constexpr uint32_t kTcSpinLimit = 1u << 24;
 constexpr uint32_t kInstrDesc = (1u << 4)           // D: FP32
@@ -137,6 +136,13 @@ __device__ __forceinline__ uint4 bf16x8(const float4& a, const float4& b) {
     return o;
 }
 
+// CTAs that share a tile's z-slices, where there are more CTAs than tiles.  A
+// tile by itself takes a CTA some 20 us, most of it MMAs one after the other: a
+// training step on one tile went from 419 to 332 us, on 64 from 462 to 403.  The
+// kernels have a body for whole tiles too: with the slices' bounds in registers
+// one on 4,096 tiles took 2.5% longer.
+__device__ __forceinline__ uint32_t tile_parts(uint32_t n) { return 4u * n <= gridDim.x ? 4u : (2u * n <= gridDim.x ? 2u : 1u); }
+
 // shared-memory footprint of one CTA for dilation DIL.  The planes lie 64
 // bytes more than their size apart, so that a voxel's two stores fall on
 // different banks.  The dilation-4 box leaves room for one CTA per SM, which
@@ -163,10 +169,10 @@ struct TcSmem {
 // dilation 2 and 4: forward 118 and 462 -> 100 and 243 us; the input gradient
 // 131 and 305 us, against 583 us with each voxel's 27 neighbours gathered into a
 // K-major A, 128 voxels at a time.
-template <int DIL, bool GRAD>
-__global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
-    lp_mid_tc_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in_,
-                     const __nv_bfloat16* __restrict__ ain, void* __restrict__ out_, int* __restrict__ err) {
+template <int DIL, bool GRAD, bool SPLIT>
+__device__ __forceinline__ void mid_tc_body(const LpGrid& G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in_,
+                                            const __nv_bfloat16* __restrict__ ain, void* __restrict__ out_,
+                                            int* __restrict__ err, int& s_abort, uint32_t (&s_nb)[2][27]) {
     using S = TcSmem<DIL>;
     constexpr int B = S::B, kThr = S::kThreads;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -174,9 +180,6 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
     unsigned char* wsm = smem + S::kBox;
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::kBox + S::kW);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kBox + S::kW + 16);
-    __shared__ int s_abort;
-    __shared__ uint32_t s_nb[2][27];  // this tile's neighbours and the next one's
-    if (G.halt && *G.halt) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     // weights: global [tap][ci][co] -> per tap a K-major B: rows = co, K = ci
@@ -198,7 +201,9 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     const uint32_t n = *G.d_nact;
-    if (warp == 1 && lane < 27 && blockIdx.x < n) s_nb[0][lane] = tile_neighbour(G, G.act_tiles[blockIdx.x], lane);
+    const uint32_t parts = SPLIT ? tile_parts(n) : 1u, all = n * parts;
+    const int nz = 8 / (int)parts;
+    if (warp == 1 && lane < 27 && blockIdx.x < all) s_nb[0][lane] = tile_neighbour(G, G.act_tiles[blockIdx.x / parts], lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -207,11 +212,12 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
     uint32_t phase = 0;
     bool pending_mma = false;
     int cur = 0;
-    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x, cur ^= 1) {
-        const uint32_t key = G.act_tiles[t];
+    for (uint32_t t = blockIdx.x; t < all; t += gridDim.x, cur ^= 1) {
+        const uint32_t key = G.act_tiles[t / parts];
+        const int z0 = (int)(t % parts) * nz, z1 = z0 + nz;  // this CTA's slices
         int ox, oy, oz;
         tile_origin_tc(key, G.D, ox, oy, oz);
-        // 1. input box, two 16-byte chunks per voxel
+        // 1. input box (of the slices: z0 .. z1 + 2 DIL), two 16-byte chunks per voxel
         auto source = [&](int e, uint32_t& sl) {  // its voxel's slot; whether there is one
             const int v = e >> 1;
             const int px = v % B - DIL, py = (v / B) % B - DIL, pz = v / (B * B) - DIL;
@@ -220,17 +226,17 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
             sl = ok ? base | rel_local(px, py, pz) : 0u;
             return ok;
         };
-        constexpr int kItems = 2 * B * B * B;
+        const int first = 2 * B * B * z0, last = 2 * B * B * (z1 + 2 * DIL);
         if (GRAD) {
             const float* in = static_cast<const float*>(in_);
-            for (int e0 = tid; e0 < kItems; e0 += 4 * kThr) {
+            for (int e0 = first + tid; e0 < last; e0 += 4 * kThr) {
                 float4 g[4][2];
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const int e = e0 + m * kThr;
                     uint32_t sl;
                     g[m][0] = g[m][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (e < kItems && source(e, sl)) {
+                    if (e < last && source(e, sl)) {
                         const float4* p = reinterpret_cast<const float4*>(in + (size_t)sl * 16 + (e & 1) * 8);
                         g[m][0] = p[0];
                         g[m][1] = p[1];
@@ -239,13 +245,13 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const int e = e0 + m * kThr;
-                    if (e < kItems)
+                    if (e < last)
                         *reinterpret_cast<uint4*>(box + (e & 1) * S::kPlane + (e >> 1) * 16) = bf16x8(g[m][0], g[m][1]);
                 }
             }
         } else {
             const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(in_);
-            for (int e = tid; e < kItems; e += kThr) {
+            for (int e = first + tid; e < last; e += kThr) {
                 uint32_t sl;
                 const bool ok = source(e, sl);
                 cp_async16(box_s + (uint32_t)((e & 1) * S::kPlane + (e >> 1) * 16), in + (size_t)sl * 16 + (e & 1) * 8, ok);
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
         tc_fence_after();
         // 2. 8 slices x 27 taps of M=64 N=16 K=16
         if (tid == 0) {
-            for (int z = 0; z < 8; ++z) {
+            for (int z = z0; z < z1; ++z) {
                 if (DIL == 4) {
                     // a descriptor holds its address in units of 16 B, and the
                     // taps' offsets are constants: an addition each
@@ -291,8 +297,8 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
             mma_commit(mbar_s);
         }
         pending_mma = true;
-        if (warp == 1 && lane < 27 && t + gridDim.x < n)
-            s_nb[cur ^ 1][lane] = tile_neighbour(G, G.act_tiles[t + gridDim.x], lane);
+        if (warp == 1 && lane < 27 && t + gridDim.x < all)
+            s_nb[cur ^ 1][lane] = tile_neighbour(G, G.act_tiles[(t + gridDim.x) / parts], lane);
         // 3. epilogue: warp w reads sub-partition w % 4 of every (warps / 4)-th slice
         const bool ok = mbar_wait(mbar_s, phase);
         if (!ok) {
@@ -304,7 +310,7 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
         phase ^= 1u;
         tc_fence_after();
         const int q = warp & 3;
-        for (int zz = warp >> 2; zz < 8; zz += kThr / 128) {
+        for (int zz = z0 + (warp >> 2); zz < z1; zz += kThr / 128) {
             float v[16];
             tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(zz * 16), v);
             if (lane < 16) {
@@ -350,6 +356,17 @@ __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
+}
+
+template <int DIL, bool GRAD>
+__global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
+    lp_mid_tc_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in,
+                     const __nv_bfloat16* __restrict__ ain, void* __restrict__ out, int* __restrict__ err) {
+    __shared__ int s_abort;
+    __shared__ uint32_t s_nb[2][27];  // a tile's neighbours and the next one's
+    if (G.halt && *G.halt) return;
+    if (tile_parts(*G.d_nact) == 1u) mid_tc_body<DIL, GRAD, false>(G, wb, in, ain, out, err, s_abort, s_nb);
+    else mid_tc_body<DIL, GRAD, true>(G, wb, in, ain, out, err, s_abort, s_nb);
 }
 
 template <int DIL, bool GRAD>
@@ -601,21 +618,19 @@ __global__ void __launch_bounds__(512) lp_in_rows_kernel(LpGrid G, const float* 
     }
 }
 
-template <int WG, int DIL>
-__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const float* __restrict__ gout,
-                                                                 const __nv_bfloat16* __restrict__ ain,
-                                                                 const float* __restrict__ d_inv_s, float sign,
-                                                                 const uint32_t* __restrict__ tiles,
-                                                                 const uint32_t* __restrict__ d_n, float* __restrict__ dw,
-                                                                 int* __restrict__ err) {
+template <int WG, int DIL, bool SPLIT>
+__device__ __forceinline__ void wgrad_body(const LpGrid& G, const float* __restrict__ gout, const __nv_bfloat16* __restrict__ ain,
+                                           const float* __restrict__ d_inv_s, float sign, const uint32_t* __restrict__ tiles,
+                                           uint32_t n, float* __restrict__ dw, int* __restrict__ err) {
     using S = WgShape<WG, DIL>;
     constexpr int B = S::B, H = S::kHalves, kStages = S::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];  // stages of the box, then B: [part][co half][512 v][8 co]
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kStages * S::kStage);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kStages * S::kStage + 32);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n = *d_n;
-    if (blockIdx.x >= n) return;
+    const uint32_t parts = SPLIT ? tile_parts(n) : 1u, all = n * parts;
+    if (blockIdx.x >= all) return;
+    const int nz = 8 / (int)parts;
     const float scale = WG == 2 ? sign / *d_inv_s : 1.0f;
     if (WG == 2)  // the columns that stay empty
         for (int e = tid; e < kStages * 2 * 512; e += kBwThreads)
@@ -639,10 +654,10 @@ __global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const
     // lane nb < 27 of every warp holds the first slot of the tile's neighbour
     // nb (a shuffle looks one up); the next tile's, and the key of the one
     // after it, are loaded a tile ahead
-    auto key_at = [&](uint32_t t) { return tiles[t < n ? t : n - 1u]; };
+    auto key_at = [&](uint32_t t) { return tiles[(t < all ? t : all - 1u) / parts]; };
     auto around = [&](uint32_t k) { return lane < 27 ? tile_neighbour(G, k, lane) : kNoTile; };
     uint32_t key = key_at(blockIdx.x), key1 = key_at(blockIdx.x + gridDim.x), nb = around(key);
-    auto gather = [&](uint32_t t, int stage) {  // the tile key of the list's t-th place; moves on to the next one
+    auto gather = [&](uint32_t t, int stage) {  // the tile key, or part of it, of place t; moves on to the next one
         unsigned char* st = smem + stage * S::kStage;
         // Gout at the tile's voxels: loads now, stores after the box's copies
         float4 g[2][2];
@@ -662,17 +677,18 @@ __global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const
         int ox, oy, oz;
         tile_origin_tc(key, G.D, ox, oy, oz);
         const uint32_t st_s = smem_s + (uint32_t)(stage * S::kStage);
-        constexpr int kItems = H * B * B * B;
+        const int z0 = (int)(t % parts) * nz;  // the box's planes that its slices take
+        const int first = H * B * B * z0, last = H * B * B * (z0 + nz + 2 * DIL);
 #pragma unroll 4
-        for (int w0 = tid - lane; w0 < kItems; w0 += kBwThreads) {  // the same for the whole warp
-            const int e = w0 + lane < kItems ? w0 + lane : kItems - 1;
+        for (int w0 = first + tid - lane; w0 < last; w0 += kBwThreads) {  // the same for the whole warp
+            const int e = w0 + lane < last ? w0 + lane : last - 1;
             const int h = e % H, v = e / H;
             const int bx = v % B, by = (v / B) % B, bz = v / (B * B);
             const int px = bx - DIL, py = by - DIL, pz = bz - DIL;
             const uint32_t base = __shfl_sync(0xffffffffu, nb, rel_neighbour(px, py, pz));
             const bool ok = base != kNoTile && ox + px < G.D.nx && oy + py < G.D.ny && oz + pz < G.D.nz;
             const uint32_t sl = ok ? base | rel_local(px, py, pz) : 0u;
-            if (w0 + lane < kItems)
+            if (w0 + lane < last)
                 cp_async16(st_s + (uint32_t)((S::row(bz, by) + h) * S::kRow + bx * 16), ain + (size_t)sl * (8 * H) + h * 8, ok);
         }
         cp_async_commit();
@@ -704,21 +720,22 @@ __global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const
     auto wait_tile = [&](uint32_t k) {
         return mbar_wait(mbar_s + 8u * (k % kStages), (k / kStages) & 1u);
     };
-    for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < all; t += gridDim.x) {
         cp_async_wait<0>();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // one decision for the whole CTA
         if (__syncthreads_or(failed)) break;
         if (tid == 0) {
             const uint32_t a_s = smem_s + (i % kStages) * S::kStage, b_s = a_s + S::kBox;
-            for (int ks = 0; ks < 32; ++ks) {
+            const int k0 = 4 * (int)(t % parts) * nz;
+            for (int ks = k0; ks < k0 + 4 * nz; ++ks) {
                 // rows y and y + DIL of slice z
                 const int z = ks >> 2, y = ((ks & 3) / DIL) * 2 * DIL + (ks & 3) % DIL;
                 const uint64_t bd = umma_desc(b_s + (uint32_t)((64 * z + 8 * y) * 16), DIL * 128, S::kPart);
                 // a descriptor holds its address in units of 16 B, and the
                 // offsets of the nine (dz, dx) are constants: an addition each
                 const uint64_t ad = umma_desc(a_s + (uint32_t)(S::row(z, y) * S::kRow), H * S::kRow, S::kRow);
-                const uint32_t add = (i > 0 || ks > 0) ? 1u : 0u;
+                const uint32_t add = (i > 0 || ks > k0) ? 1u : 0u;
 #pragma unroll
                 for (int j = 0; j < 9; ++j)
                     mma_f16(tmem + (uint32_t)(S::kN * j), ad + (uint64_t)((S::row(DIL * (j / 3), 0) * S::kRow) / 16 + DIL * (j % 3)), bd,
@@ -727,7 +744,7 @@ __global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const
             mma_commit(mbar_s + 8u * (i % kStages));
         }
         ++i;
-        if (t + gridDim.x < n) {
+        if (t + gridDim.x < all) {
             // the stage is that of the tile kStages before: its MMAs have to be done
             if (i >= (uint32_t)kStages && !wait_tile(i - kStages)) failed = true;
             if (!__any_sync(0xffffffffu, failed)) gather(t + gridDim.x, (int)(i % kStages));
@@ -782,6 +799,18 @@ __global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const
     __syncthreads();
     tc_fence_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kCols) : "memory");
+}
+
+template <int WG, int DIL>
+__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const float* __restrict__ gout,
+                                                                 const __nv_bfloat16* __restrict__ ain,
+                                                                 const float* __restrict__ d_inv_s, float sign,
+                                                                 const uint32_t* __restrict__ tiles,
+                                                                 const uint32_t* __restrict__ d_n, float* __restrict__ dw,
+                                                                 int* __restrict__ err) {
+    const uint32_t n = *d_n;
+    if (tile_parts(n) == 1u) wgrad_body<WG, DIL, false>(G, gout, ain, d_inv_s, sign, tiles, n, dw, err);
+    else wgrad_body<WG, DIL, true>(G, gout, ain, d_inv_s, sign, tiles, n, dw, err);
 }
 
 template <int WG, int DIL>
