@@ -37,6 +37,7 @@ WORKLOAD = ("dam-break 256^3 voxels (cell 1/256), block 0.5x0.5x1, 8 jittered pa
 # matvec+pAp 9 B, x/r/z update with r.z 28 B, direction update 12 B
 PCG_BYTES_PER_VOXEL = 49.0
 RESIDENT_TILES = 88  # tiles per SM that the resident Jacobi-PCG solve holds
+EXCHANGE_US = 2.6    # its grid-wide exchange on 148 CTAs: what an iteration cannot do without
 # one learned multilevel FCG iteration on the fine level: direction+matvec and
 # update 49 B, V-cycle down (code, r in; t, coarse r out) 9.5 B and up (code,
 # r, t in; z out) 12.5 B, plus q in 4 B for the FCG dot products the up
@@ -574,13 +575,21 @@ def main():
     resident = fluid_tiles <= RESIDENT_TILES * torch.cuda.get_device_properties(dev).multi_processor_count
     if c5 or resident:
         traffic = None  # the ncu traffic figure covers the two-kernel Jacobi-PCG iteration only
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic,
-                "kernel": ("learned multilevel FCG iteration (direction+matvec, update, V-cycle with the FCG dot fused)" if c5 else
-                           "pcg iteration (resident kernel: vectors on the chip, so the fraction of the streamed minimum passes 1)" if resident else
-                           "pcg iteration (matvec+pAp, x/r update with r.r and r.z, direction)"),
-                "algorithmic_bytes": "%d B per active voxel per iteration x %d voxels" % (per_voxel, voxels),
-                "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6650 GB/s"}
+    if resident and not c5:
+        # the vectors stay on the chip: no HBM bound; the iteration's floor is its exchange
+        roofline = {"bound": "latency", "achieved": 1e3 * t_iter_ms, "peak": EXCHANGE_US, "unit": "us per iteration",
+                    "frac": EXCHANGE_US / (1e3 * t_iter_ms), "traffic": None,
+                    "kernel": "pcg iteration (resident kernel)",
+                    "algorithmic_bytes": "none from HBM; a solver that streams its vectors takes %d B per active voxel per "
+                                         "iteration x %d voxels" % (per_voxel, voxels),
+                    "peak_source": "measured: two-hop exchange of five sums over 148 CTAs"}
+    else:
+        roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                    "traffic": traffic,
+                    "kernel": ("learned multilevel FCG iteration (direction+matvec, update, V-cycle with the FCG dot fused)" if c5
+                               else "pcg iteration (matvec+pAp, x/r update with r.r and r.z, direction)"),
+                    "algorithmic_bytes": "%d B per active voxel per iteration x %d voxels" % (per_voxel, voxels),
+                    "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback 6650 GB/s"}
 
     # the particle-stage metric: binning, P2G and G2P/advection only
     part_keys = ["keys", "sort", "gather", "segment_heads", "grid_clear", "p2g", "g2p_advect"]
@@ -600,6 +609,8 @@ def main():
         "pcg_iterations": per_voxel * voxels * it_step,
         "projection": 29.0 * voxels,
     }
+    if resident and not c5:
+        del stage_bytes["pcg_iterations"]  # nothing streams
     stages_gbs = {}
     for k, b in stage_bytes.items():
         if stages.get(k, 0.0) > 0.0:

@@ -252,7 +252,8 @@ __global__ void __launch_bounds__(kEdgeThreads) lp_out_kernel(LpGrid G, const __
 // only tests the grid bounds.
 // A pass is four kernels of a few microseconds whose latency is all they
 // cost: what does not depend on the previous kernel (weights, the voxels'
-// cells, the tensor memory) is fetched before pdl_wait(), beside it, and a
+// cells) is fetched before pdl_wait(), beside it (not the tensor memory: a
+// kernel's CTAs could hold what the one they wait for has yet to take), and a
 // thread's gathers are independent loads in flight together.  With both after
 // the wait and a tile lookup per tap, an FCG iteration on 864 and 4,096 tiles
 // took 89 and 118 us, now 86 and 115 us.
