@@ -55,7 +55,7 @@ struct flip_engine {
     double* pt[6] = {};  // gather targets
     uint32_t *ytable = nullptr, *counts = nullptr, *masks = nullptr, *node_voxels = nullptr;
     uint64_t node_cap = 0;
-    double* getmax_buf = nullptr;
+    double *getmax_n = nullptr, *getmax_vox = nullptr;  // block maxima of particle and of voxel arrays
     uint64_t vox_cap = 0;
     uint32_t voxels = 0;
     uint32_t* voxel_ids = nullptr;
@@ -319,10 +319,10 @@ static void free_arena(flip_engine* e) {
     e->arena_bytes = 0;
 }
 static void free_ref_voxels(flip_engine* e) {
-    void* ps[] = {e->voxel_ids, e->solids, e->ux, e->uy, e->uz, e->divU, e->p, e->res};
+    void* ps[] = {e->voxel_ids, e->solids, e->ux, e->uy, e->uz, e->divU, e->p, e->res, e->getmax_vox};
     for (void* q : ps) if (q) cudaFree(q);
     e->voxel_ids = nullptr; e->solids = nullptr;
-    e->ux = e->uy = e->uz = e->divU = e->p = e->res = nullptr;
+    e->ux = e->uy = e->uz = e->divU = e->p = e->res = e->getmax_vox = nullptr;
     e->vox_cap = 0;
 }
 
@@ -369,7 +369,7 @@ extern "C" int flip_set_domain(flip_engine* e, double nx, double ny, double nz, 
         add((void**)&e->counts, 4 * e->node_cap);
         add((void**)&e->node_voxels, 4 * e->node_cap);
         add((void**)&e->masks, 64 * e->node_cap);
-        add((void**)&e->getmax_buf, 16 * (n / 512 + 2));
+        add((void**)&e->getmax_n, flip_ref_getmax_scratch_bytes(n));
     } else {
         uint64_t NX = 4ull * x, NY = 4ull * y, NZ = 4ull * z;
         if (NX % 8 || NY % 8 || NZ % 8)
@@ -612,6 +612,7 @@ static int ensure_voxels(flip_engine* e, uint64_t need) {
     E_CUDA(cudaMalloc((void**)&e->solids, cap));
     double** d[6] = {&e->ux, &e->uy, &e->uz, &e->divU, &e->p, &e->res};
     for (double** q : d) E_CUDA(cudaMalloc((void**)q, 8 * cap));
+    E_CUDA(cudaMalloc((void**)&e->getmax_vox, flip_ref_getmax_scratch_bytes(cap)));
     e->vox_cap = cap;
     return FLIP_OK;
 }
@@ -650,10 +651,10 @@ static int ref_p2g_stage(flip_engine* e) {
                           e->node_voxels, e->voxel_ids, e->solids, e->grid, e->ux, e->uy, e->uz, e->stream);
 }
 
-// CudaVec<double>::getMax (cudaVec.cu:205-233) with the reference's reduction
-static int ref_getmax(flip_engine* e, const double* a, uint64_t n, bool absolute, double* out) {
-    double* b0 = e->getmax_buf;
-    double* b1 = e->getmax_buf + (e->n / 512 + 2);
+// CudaVec<double>::getMax (cudaVec.cu:205-233) with the reference's reduction;
+// scratch: flip_ref_getmax_scratch_bytes(n)
+static int ref_getmax(flip_engine* e, const double* a, uint64_t n, double* scratch, bool absolute, double* out) {
+    double *b0 = scratch, *b1 = scratch + (n / 512 + 2);
     E_TRY(ref_launch_getmax_level(n, a, b0, absolute ? 1 : 0, e->stream));
     for (uint64_t i = n / 512 + 1; i > 1; i = i / 512 + 1) {
         E_TRY(ref_launch_getmax_level(i, b0, b1, absolute ? 1 : 0, e->stream));
@@ -669,9 +670,9 @@ static int ref_getmax(flip_engine* e, const double* a, uint64_t n, bool absolute
 
 static int ref_courant_dt(flip_engine* e, double* dt) {
     double a, b, c;
-    E_TRY(ref_getmax(e, e->pd[3], e->n, true, &a));
-    E_TRY(ref_getmax(e, e->pd[4], e->n, true, &b));
-    E_TRY(ref_getmax(e, e->pd[5], e->n, true, &c));
+    E_TRY(ref_getmax(e, e->pd[3], e->n, e->getmax_n, true, &a));
+    E_TRY(ref_getmax(e, e->pd[4], e->n, e->getmax_n, true, &b));
+    E_TRY(ref_getmax(e, e->pd[5], e->n, e->getmax_n, true, &c));
     double maxVel = std::max(std::fabs(a), std::max(std::fabs(b), std::fabs(c)));
     double voxelSize = (double)e->grid.cellSize / (8.0 - 2.0 * std::floor(2.0));
     *dt = 0.7 * (voxelSize / maxVel);
@@ -704,7 +705,7 @@ static int ref_gs_solve(flip_engine* e, double dt, double threshold, uint32_t ma
         it += chunk;
         if (first % 1024 == 0) {
             prevR = maxR;
-            E_TRY(ref_getmax(e, e->res, e->voxels, true, &maxR));
+            E_TRY(ref_getmax(e, e->res, e->voxels, e->getmax_vox, true, &maxR));
         }
         if (it == max_iter || (std::fabs(prevR - maxR) < threshold / 1000 && maxR > threshold)) break;
     }
