@@ -169,46 +169,18 @@ struct TcSmem {
 // dilation 2 and 4: forward 118 and 462 -> 100 and 243 us; the input gradient
 // 131 and 305 us, against 583 us with each voxel's 27 neighbours gathered into a
 // K-major A, 128 voxels at a time.
+// mid_tc_tiles: the tiles (SPLIT: parts of tiles) of a CTA.
 template <int DIL, bool GRAD, bool SPLIT>
-__device__ __forceinline__ void mid_tc_body(const LpGrid& G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in_,
-                                            const __nv_bfloat16* __restrict__ ain, void* __restrict__ out_,
-                                            int* __restrict__ err, int& s_abort, uint32_t (&s_nb)[2][27]) {
+__device__ __forceinline__ void mid_tc_tiles(const LpGrid& G, const void* __restrict__ in_, const __nv_bfloat16* __restrict__ ain,
+                                             void* __restrict__ out_, int* __restrict__ err, uint32_t n, uint32_t tmem,
+                                             unsigned char* smem, int& s_abort, uint32_t (&s_nb)[2][27]) {
     using S = TcSmem<DIL>;
     constexpr int B = S::B, kThr = S::kThreads;
-    extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* box = smem;
-    unsigned char* wsm = smem + S::kBox;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::kBox + S::kW);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kBox + S::kW + 16);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    // weights: global [tap][ci][co] -> per tap a K-major B: rows = co, K = ci
-    // (GRAD: rows = ci, K = co)
-    for (int e = tid; e < 27 * 256; e += kThr) {
-        const int tap = e >> 8, ci = (e >> 4) & 15, co = e & 15;
-        const int row = GRAD ? ci : co, k = GRAD ? co : ci;
-        *reinterpret_cast<__nv_bfloat16*>(wsm + tap * 512 + (k >> 3) * 256 + row * 16 + (k & 7) * 2) = wb[e];
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_abort = 0;
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(kTcCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    const uint32_t n = *G.d_nact;
     const uint32_t parts = SPLIT ? tile_parts(n) : 1u, all = n * parts;
     const int nz = 8 / (int)parts;
-    if (warp == 1 && lane < 27 && blockIdx.x < all) s_nb[0][lane] = tile_neighbour(G, G.act_tiles[blockIdx.x / parts], lane);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t box_s = smem_u32(box), w_s = smem_u32(wsm), mbar_s = smem_u32(mbar);
+    const uint32_t box_s = smem_u32(box), w_s = box_s + S::kBox, mbar_s = w_s + S::kW;
     uint32_t phase = 0;
     bool pending_mma = false;
     int cur = 0;
@@ -354,19 +326,52 @@ __device__ __forceinline__ void mid_tc_body(const LpGrid& G, const __nv_bfloat16
         if (pending_mma) mbar_wait(mbar_s, phase);
         __syncthreads();
     }
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
 }
 
 template <int DIL, bool GRAD>
 __global__ void __launch_bounds__(TcSmem<DIL>::kThreads)
     lp_mid_tc_kernel(LpGrid G, const __nv_bfloat16* __restrict__ wb, const void* __restrict__ in,
                      const __nv_bfloat16* __restrict__ ain, void* __restrict__ out, int* __restrict__ err) {
+    using S = TcSmem<DIL>;
+    constexpr int kThr = S::kThreads;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char* wsm = smem + S::kBox;
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::kBox + S::kW);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kBox + S::kW + 16);
     __shared__ int s_abort;
-    __shared__ uint32_t s_nb[2][27];  // a tile's neighbours and the next one's
+    __shared__ uint32_t s_nb[2][27];  // this tile's neighbours and the next one's
     if (G.halt && *G.halt) return;
-    if (tile_parts(*G.d_nact) == 1u) mid_tc_body<DIL, GRAD, false>(G, wb, in, ain, out, err, s_abort, s_nb);
-    else mid_tc_body<DIL, GRAD, true>(G, wb, in, ain, out, err, s_abort, s_nb);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    // weights: global [tap][ci][co] -> per tap a K-major B: rows = co, K = ci
+    // (GRAD: rows = ci, K = co)
+    for (int e = tid; e < 27 * 256; e += kThr) {
+        const int tap = e >> 8, ci = (e >> 4) & 15, co = e & 15;
+        const int row = GRAD ? ci : co, k = GRAD ? co : ci;
+        *reinterpret_cast<__nv_bfloat16*>(wsm + tap * 512 + (k >> 3) * 256 + row * 16 + (k & 7) * 2) = wb[e];
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(kTcCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    const uint32_t n = *G.d_nact, parts = tile_parts(n);
+    if (warp == 1 && lane < 27 && blockIdx.x < n * parts)
+        s_nb[0][lane] = tile_neighbour(G, G.act_tiles[blockIdx.x / parts], lane);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    if (parts == 1u) mid_tc_tiles<DIL, GRAD, false>(G, in, ain, out, err, n, tmem, smem, s_abort, s_nb);
+    else mid_tc_tiles<DIL, GRAD, true>(G, in, ain, out, err, n, tmem, smem, s_abort, s_nb);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols) : "memory");
 }
 
 template <int DIL, bool GRAD>
