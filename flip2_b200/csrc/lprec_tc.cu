@@ -138,9 +138,9 @@ __device__ __forceinline__ uint4 bf16x8(const float4& a, const float4& b) {
 
 // CTAs that share a tile's z-slices, where there are more CTAs than tiles.  A
 // tile by itself takes a CTA some 20 us, most of it MMAs one after the other: a
-// training step on one tile went from 419 to 332 us, on 64 from 462 to 403.  The
-// kernels have a body for whole tiles too: with the slices' bounds in registers
-// one on 4,096 tiles took 2.5% longer.
+// training step on one tile went from 419 to 332 us, on 64 from 462 to 403.  Whole
+// tiles have a form of their own: with the slices' bounds in registers a step on
+// 4,096 tiles took 2.5% longer.
 __device__ __forceinline__ uint32_t tile_parts(uint32_t n) { return 4u * n <= gridDim.x ? 4u : (2u * n <= gridDim.x ? 2u : 1u); }
 
 // shared-memory footprint of one CTA for dilation DIL.  The planes lie 64
@@ -623,17 +623,23 @@ __global__ void __launch_bounds__(512) lp_in_rows_kernel(LpGrid G, const float* 
     }
 }
 
+// SPLIT: a tile's K-steps shared as tile_parts() says (a kernel of its own:
+// with both forms in one, whole tiles of the input layer took 42 instead of 37 us
+// on 343 tiles)
 template <int WG, int DIL, bool SPLIT>
-__device__ __forceinline__ void wgrad_body(const LpGrid& G, const float* __restrict__ gout, const __nv_bfloat16* __restrict__ ain,
-                                           const float* __restrict__ d_inv_s, float sign, const uint32_t* __restrict__ tiles,
-                                           uint32_t n, float* __restrict__ dw, int* __restrict__ err) {
+__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const float* __restrict__ gout,
+                                                                 const __nv_bfloat16* __restrict__ ain,
+                                                                 const float* __restrict__ d_inv_s, float sign,
+                                                                 const uint32_t* __restrict__ tiles,
+                                                                 const uint32_t* __restrict__ d_n, float* __restrict__ dw,
+                                                                 int* __restrict__ err) {
     using S = WgShape<WG, DIL>;
     constexpr int B = S::B, H = S::kHalves, kStages = S::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];  // stages of the box, then B: [part][co half][512 v][8 co]
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kStages * S::kStage);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kStages * S::kStage + 32);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t parts = SPLIT ? tile_parts(n) : 1u, all = n * parts;
+    const uint32_t n = *d_n, parts = SPLIT ? tile_parts(n) : 1u, all = n * parts;
     if (blockIdx.x >= all) return;
     const int nz = 8 / (int)parts;
     const float scale = WG == 2 ? sign / *d_inv_s : 1.0f;
@@ -806,23 +812,11 @@ __device__ __forceinline__ void wgrad_body(const LpGrid& G, const float* __restr
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kCols) : "memory");
 }
 
-template <int WG, int DIL>
-__global__ void __launch_bounds__(kBwThreads) lp_tc_wgrad_kernel(LpGrid G, const float* __restrict__ gout,
-                                                                 const __nv_bfloat16* __restrict__ ain,
-                                                                 const float* __restrict__ d_inv_s, float sign,
-                                                                 const uint32_t* __restrict__ tiles,
-                                                                 const uint32_t* __restrict__ d_n, float* __restrict__ dw,
-                                                                 int* __restrict__ err) {
-    const uint32_t n = *d_n;
-    if (tile_parts(n) == 1u) wgrad_body<WG, DIL, false>(G, gout, ain, d_inv_s, sign, tiles, n, dw, err);
-    else wgrad_body<WG, DIL, true>(G, gout, ain, d_inv_s, sign, tiles, n, dw, err);
-}
-
-template <int WG, int DIL>
-static int launch_wgrad_tc(const LpGrid& G, const float* gout, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
+template <int WG, int DIL, bool SPLIT>
+static int launch_wgrad_form(const LpGrid& G, const float* gout, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
                             const uint32_t* tiles, const uint32_t* d_n, float* dw, int* err, int sms, cudaStream_t st) {
     using S = WgShape<WG, DIL>;
-    const auto kernel = lp_tc_wgrad_kernel<WG, DIL>;
+    const auto kernel = lp_tc_wgrad_kernel<WG, DIL, SPLIT>;
     static bool attr_set = false;  // per process; the attribute is per function
     if (!attr_set) {
         FLIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
@@ -831,6 +825,13 @@ static int launch_wgrad_tc(const LpGrid& G, const float* gout, const __nv_bfloat
     kernel<<<sms, kBwThreads, S::kBytes, st>>>(G, gout, ain, d_inv_s, sign, tiles, d_n, dw, err);
     FLIP_CUDA_TRY(cudaGetLastError());
     return FLIP_OK;
+}
+// shared tiles where a box has no more of them than half the CTAs
+template <int WG, int DIL>
+static int launch_wgrad_tc(const LpGrid& G, const float* gout, const __nv_bfloat16* ain, const float* d_inv_s, float sign,
+                           const uint32_t* tiles, const uint32_t* d_n, float* dw, int* err, int sms, cudaStream_t st) {
+    const auto launch = 2ll * G.D.tx * G.D.ty * G.D.tz <= sms ? launch_wgrad_form<WG, DIL, true> : launch_wgrad_form<WG, DIL, false>;
+    return launch(G, gout, ain, d_inv_s, sign, tiles, d_n, dw, err, sms, st);
 }
 int lp_in_wgrad_tc(const LpGrid& G, int dil, const float* gout, const float* d_inv_s, void* rows, float* dw, int* err, int sms,
                    cudaStream_t st) {
